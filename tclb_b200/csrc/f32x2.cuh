@@ -56,8 +56,50 @@ __device__ __forceinline__ F2& operator*=(F2& x, F2 y) { return x = F2(x * y); }
 __device__ __forceinline__ F2& operator+=(F2& x, F2Prod p) { return x = p + x; }
 __device__ __forceinline__ F2& operator-=(F2& x, F2Prod p) { return x = x - p; }
 
+// One value with the operators of F2, every operation and contraction spelled
+// out: collision code instantiated with X1<float> does on one node exactly
+// what F2 does on each lane, and any two kernels that inline it round alike
+// (the compiler is left no choice of which product of a sum to fuse).
+__device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
+
+template <class R>
+struct X1 {
+  R v;
+  X1() = default;
+  __device__ __forceinline__ X1(double x) : v((R)x) {}
+  __device__ __forceinline__ X1(float x) : v((R)x) {}
+  __device__ __forceinline__ X1(int x) : v((R)x) {}
+};
+template <class R>
+struct X1Prod {
+  R a, b;
+  __device__ __forceinline__ operator X1<R>() const { return X1<R>(mul_rn(a, b)); }
+};
+#define X1_OP template <class R> __device__ __forceinline__
+X1_OP X1<R> val(X1Prod<R> p) { return X1<R>(mul_rn(p.a, p.b)); }
+X1_OP X1Prod<R> operator*(X1<R> x, X1<R> y) { return {x.v, y.v}; }
+X1_OP X1Prod<R> operator*(X1Prod<R> p, X1<R> y) { return {val(p).v, y.v}; }
+X1_OP X1Prod<R> operator*(X1<R> x, X1Prod<R> p) { return {x.v, val(p).v}; }
+X1_OP X1<R> operator+(X1<R> x, X1<R> y) { return X1<R>(add_rn(x.v, y.v)); }
+X1_OP X1<R> operator-(X1<R> x, X1<R> y) { return X1<R>(add_rn(x.v, -y.v)); }
+X1_OP X1<R> operator-(X1<R> x) { return X1<R>(-x.v); }
+X1_OP X1<R> operator+(X1Prod<R> p, X1<R> c) { return X1<R>(fma_rn(p.a, p.b, c.v)); }
+X1_OP X1<R> operator+(X1<R> c, X1Prod<R> p) { return X1<R>(fma_rn(p.a, p.b, c.v)); }
+X1_OP X1<R> operator-(X1Prod<R> p, X1<R> c) { return X1<R>(fma_rn(p.a, p.b, -c.v)); }
+X1_OP X1<R> operator-(X1<R> c, X1Prod<R> p) { return X1<R>(fma_rn(-p.a, p.b, c.v)); }
+X1_OP X1<R> operator+(X1Prod<R> p, X1Prod<R> q) { return X1<R>(fma_rn(p.a, p.b, val(q).v)); }
+X1_OP X1<R> operator-(X1Prod<R> p, X1Prod<R> q) { return X1<R>(fma_rn(p.a, p.b, -val(q).v)); }
+#undef X1_OP
+
 // 1 / x per lane (IEEE division, as R(1) / x in the scalar code)
 __device__ __forceinline__ F2 recip(F2 x) { return F2(1.0f / x.v.x, 1.0f / x.v.y); }
+template <class R>
+__device__ __forceinline__ X1<R> recip(X1<R> x) { return X1<R>(R(1) / x.v); }
 template <class R>
 __device__ __forceinline__ R recip(R x) { return R(1) / x; }
 

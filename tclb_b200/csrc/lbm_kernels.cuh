@@ -120,7 +120,9 @@ struct D2Q9 {
   static constexpr int PAIR_THREADS = 256, PAIR_MIN_BLOCKS = 4;  // <= 64 registers
   static constexpr int BATCH_MIN_BLOCKS = 6;  // one-tile batch kernel: <= 40 registers
   template <class R>
-  __host__ __device__ static void derived(const R*, R* k) { k[0] = k[1] = k[2] = k[3] = R(0); }
+  __host__ __device__ static void derived(const R*, R* k) {
+    k[0] = k[1] = k[2] = k[3] = R(0);
+  }
   __host__ __device__ static constexpr int ex(int i) { return (i == 1 || i == 5 || i == 8) ? 1 : ((i == 3 || i == 6 || i == 7) ? -1 : 0); }
   __host__ __device__ static constexpr int ey(int i) { return (i == 2 || i == 5 || i == 6) ? 1 : ((i == 4 || i == 7 || i == 8) ? -1 : 0); }
   __host__ __device__ static constexpr int ez(int) { return 0; }
@@ -189,20 +191,68 @@ struct D2Q9 {
     f[8] = R(1.0 / 36.0) * (a + r1 - r2 - R(3) * r5 - R(2) * r6 + R(2) * r7);
   }
 
+  // The MRT update, for value type V (X1 for one node, F2 for two), on the sums
+  // and differences of opposite populations: the moments even under e -> -e
+  // (rho, 3x^2-1, 3y^2-1, 3xy and the fourth-order one) need the sums only,
+  // the odd ones (J and the third-order ones) the differences, and so back:
+  // about 85 operations instead of 150 with each moment from all populations.
+  // Leaves rho and J before the force for the Globals. The rest population
+  // closes the mass exactly. With DEV the values are deviations g = f - w:
+  // the weights' moments are all zero but the density (1), so rho is rho - 1
+  // in every linear term and the true density only divides J.
+  template <bool DEV, class V, class AR>
+  __device__ __forceinline__ static void relax(V (&f)[Q], const AR& a, V& rho, V& jx, V& jy) {
+    const V s1 = f[1] + f[3], s2 = f[2] + f[4], s5 = f[5] + f[7], s6 = f[6] + f[8];
+    const V d1 = f[1] - f[3], d2 = f[2] - f[4], d5 = f[5] - f[7], d6 = f[6] - f[8];
+    const V s12 = s1 + s2, d = s5 + s6, p56 = d5 + d6, q56 = d5 - d6;
+    rho = f[0] + s12 + d;
+    jx = d1 + q56;
+    jy = d2 + p56;
+    const V rho_t = DEV ? rho + V(1) : rho;
+    const V i3 = V(3) * recip(rho_t);
+    const V ux = i3 * jx, uy = i3 * jy;  // 3 u
+    V fx = jx, fy = jy;  // J with the force: J + rho G
+    const V gx = V(a.s[d2q9::S_GravitationX]), gy = V(a.s[d2q9::S_GravitationY]);
+    fx = gx * rho_t + fx;
+    fy = gy * rho_t + fy;
+    // relaxed moments plus equilibrium at J + rho G: S (m - m_eq(J)) + m_eq(J +
+    // rho G), where m_eq(J + rho G) - m_eq(J) is linear in G (jx'^2 / rho - jx^2 /
+    // rho = G (jx + jx'))
+    const V S2 = V(a.s[d2q9::S_S2]), S3 = V(a.s[d2q9::S_S3]), S4 = V(a.s[d2q9::S_S4]);
+    const V X = ux * jx, Y = uy * jy, XY = ux * jy;  // 3 J_a J_b / rho
+    const V g3x = V(3) * gx, g3y = V(3) * gy;
+    const V m3 = V(3) * (s1 + d) - rho, m4 = V(3) * (s2 + d) - rho;
+    const V q3 = S2 * (m3 - X) + (g3x * (jx + fx) + X);
+    const V q4 = S2 * (m4 - Y) + (g3y * (jy + fy) + Y);
+    const V q5 = S2 * (V(3) * (s5 - s6) - XY) + (g3x * fy + (g3y * jx + XY));
+    const V t6 = S3 * (V(3) * p56 - jy), t7 = S3 * (V(3) * q56 - jx), t8 = S4 * (V(3) * (d - s12) + rho);
+    const V b = V(1.0 / 9.0) * rho - V(1.0 / 18.0) * t8;
+    const V E1 = V(1.0 / 9.0) * q3 + (b - V(1.0 / 18.0) * q4), E2 = V(1.0 / 9.0) * q4 + (b - V(1.0 / 18.0) * q3);
+    const V c = V(1.0 / 36.0) * ((q3 + q4) + (rho + t8));
+    const V E5 = c + V(1.0 / 12.0) * q5, E6 = c - V(1.0 / 12.0) * q5;
+    const V O1 = V(2) * fx - t7, O2 = V(2) * fy - t6, A = fx + t7, B = fy + t6;
+    const V O5 = B + A, O6 = B - A;
+    f[0] = rho - V(2) * ((E1 + E2) + (E5 + E6));
+    f[1] = E1 + V(1.0 / 6.0) * O1;
+    f[3] = E1 - V(1.0 / 6.0) * O1;
+    f[2] = E2 + V(1.0 / 6.0) * O2;
+    f[4] = E2 - V(1.0 / 6.0) * O2;
+    f[5] = E5 + V(1.0 / 12.0) * O5;
+    f[7] = E5 - V(1.0 / 12.0) * O5;
+    f[6] = E6 + V(1.0 / 12.0) * O6;
+    f[8] = E6 - V(1.0 / 12.0) * O6;
+  }
+
   template <class R, bool G>
   __device__ __forceinline__ static void mrt(R (&f)[Q], flag_t fl, const Args<R, NSET>& a, R* g, const R* zs) {
-    const R d = f[5] + f[6] + f[7] + f[8];
-    const R rho = f[0] + f[1] + f[2] + f[3] + f[4] + d;
-    R jx = f[1] - f[3] + f[5] - f[6] - f[7] + f[8];
-    R jy = f[2] - f[4] + f[5] + f[6] - f[7] - f[8];
-    R m3 = -f[0] + R(2) * (f[1] + f[3]) - f[2] - f[4] + R(2) * d;
-    R m4 = -f[0] - f[1] - f[3] + R(2) * (f[2] + f[4]) + R(2) * d;
-    R m5 = R(3) * (f[5] - f[6] + f[7] - f[8]);
-    R m6 = f[4] - f[2] + R(2) * (f[5] + f[6] - f[7] - f[8]);
-    R m7 = f[3] - f[1] + R(2) * (f[5] - f[6] - f[7] + f[8]);
-    R m8 = f[0] - R(2) * (f[1] + f[2] + f[3] + f[4]) + R(4) * d;
-    const R irho = R(1) / rho;
+    X1<R> v[Q], xr, xx, xy;
+#pragma unroll
+    for (int i = 0; i < Q; i++) v[i] = X1<R>(f[i]);
+    relax<false>(v, a, xr, xx, xy);
+#pragma unroll
+    for (int i = 0; i < Q; i++) f[i] = v[i].v;
     if (G) {  // d2q9/Dynamics.c.Rt:228-246 (pre-relaxation rho, J)
+      const R rho = xr.v, jx = xx.v, jy = xy.v;
       const unsigned obj = fl & d2q9::OBJECTIVE;
       if (obj) {
         const R usq = (jx * jx + jy * jy) / (rho * rho);
@@ -212,19 +262,6 @@ struct D2Q9 {
         else if (obj == d2q9::Inlet) { glob(g, d2q9::G_InletFlux, flux, zs); glob(g, d2q9::G_PressureLoss, pl, zs); }
       }
     }
-    const R S2 = a.s[d2q9::S_S2], S3 = a.s[d2q9::S_S3], S4 = a.s[d2q9::S_S4];
-    m3 = S2 * (m3 - R(3) * jx * jx * irho);
-    m4 = S2 * (m4 - R(3) * jy * jy * irho);
-    m5 = S2 * (m5 - R(3) * jx * jy * irho);
-    m6 = S3 * m6;
-    m7 = S3 * m7;
-    m8 = S4 * m8;
-    jx = jx + a.s[d2q9::S_GravitationX] * rho;
-    jy = jy + a.s[d2q9::S_GravitationY] * rho;
-    m3 += R(3) * jx * jx * irho;
-    m4 += R(3) * jy * jy * irho;
-    m5 += R(3) * jx * jy * irho;
-    from_moments(f, rho, jx, jy, m3, m4, m5, m6, m7, m8);
   }
 
   template <class R, bool G>
@@ -256,13 +293,8 @@ struct D2Q9 {
   }
 
   // Two nodes with one packed collision (plain iterations): boundaries per
-  // node, then the MRT update of mrt() on both lanes; a lane whose node does
-  // not collide keeps its values (pair_update_store parks them). With DEV the
-  // values are deviations g = f - w: the weights' MRT moments are all zero
-  // but the density (1), so the moments of g are those of f with rho - 1,
-  // which enters the linear terms (from_moments is linear, its rho part
-  // weighted by w), while the quadratic equilibrium terms and the force use
-  // the true density.
+  // node, then relax() on both lanes; a lane whose node does not collide
+  // keeps its values (pair_update_store parks them).
   __device__ __forceinline__ static bool collides(flag_t fl) { return (fl & d2q9::MRT) != 0; }
   __device__ __forceinline__ static bool has_boundary(flag_t fl) { return (fl & d2q9::BOUNDARY) != 0; }
   template <class R, class AR>
@@ -271,32 +303,8 @@ struct D2Q9 {
   }
   template <bool DEV, class AR>
   __device__ __forceinline__ static void collide_pair(F2 (&f)[Q], flag_t, flag_t, const AR& a) {
-    const F2 d = f[5] + f[6] + f[7] + f[8];
-    const F2 rho = f[0] + f[1] + f[2] + f[3] + f[4] + d;  // rho - 1 with DEV
-    F2 jx = f[1] - f[3] + f[5] - f[6] - f[7] + f[8];
-    F2 jy = f[2] - f[4] + f[5] + f[6] - f[7] - f[8];
-    F2 m3 = -f[0] + F2(2.0f) * (f[1] + f[3]) - f[2] - f[4] + F2(2.0f) * d;
-    F2 m4 = -f[0] - f[1] - f[3] + F2(2.0f) * (f[2] + f[4]) + F2(2.0f) * d;
-    F2 m5 = F2(3.0f) * (f[5] - f[6] + f[7] - f[8]);
-    F2 m6 = f[4] - f[2] + F2(2.0f) * (f[5] + f[6] - f[7] - f[8]);
-    F2 m7 = f[3] - f[1] + F2(2.0f) * (f[5] - f[6] - f[7] + f[8]);
-    F2 m8 = f[0] - F2(2.0f) * (f[1] + f[2] + f[3] + f[4]) + F2(4.0f) * d;
-    const F2 rho_t = DEV ? rho + F2(1.0f) : rho;  // true density
-    const F2 irho = recip(rho_t);
-    const F2 S2((float)a.s[d2q9::S_S2]), S3((float)a.s[d2q9::S_S3]), S4((float)a.s[d2q9::S_S4]);
-    const F2 gx((float)a.s[d2q9::S_GravitationX]), gy((float)a.s[d2q9::S_GravitationY]);
-    m3 = S2 * (m3 - F2(3.0f) * jx * jx * irho);
-    m4 = S2 * (m4 - F2(3.0f) * jy * jy * irho);
-    m5 = S2 * (m5 - F2(3.0f) * jx * jy * irho);
-    m6 = S3 * m6;
-    m7 = S3 * m7;
-    m8 = S4 * m8;
-    jx = jx + gx * rho_t;
-    jy = jy + gy * rho_t;
-    m3 += F2(3.0f) * jx * jx * irho;
-    m4 += F2(3.0f) * jy * jy * irho;
-    m5 += F2(3.0f) * jx * jy * irho;
-    from_moments(f, rho, jx, jy, m3, m4, m5, m6, m7, m8);
+    F2 rho, jx, jy;
+    relax<DEV>(f, a, rho, jx, jy);
   }
   template <bool DEV, class AR>
   __device__ __forceinline__ static void collide_pair_lanes(F2 (&)[Q], bool, bool, const AR&) {}
@@ -1123,6 +1131,58 @@ struct Pack16<StoreBF16<SH>> {
   }
 };
 
+// Boundaries and collision of two neighbouring nodes held packed, as pulled
+// (SHIFTED: as deviations f - w).
+template <class M, bool SHIFTED, bool LANES, class AR>
+__device__ __forceinline__ void pair_update(F2 (&f2)[M::Q], flag_t fla, flag_t flb, const AR& a) {
+  // Values stay packed (node x, node x+1). A node with a boundary type has
+  // its lane taken out, updated by the scalar boundary code and put back;
+  // then one packed FP32x2 collision serves both nodes, so bulk and
+  // boundary pairs do not diverge in the collision.
+  // With shifted storage the packed values stay deviations g = f - w
+  // (the collision works on them directly); the scalar boundary code sees f.
+  constexpr float SH = SHIFTED ? 1.0f : 0.0f;
+  if (M::has_boundary(fla)) {
+    float t[M::Q];
+#pragma unroll
+    for (int i = 0; i < M::Q; i++) t[i] = f2[i].v.x + SH * (float)M::w(i);
+    M::pre_collision(t, fla, a);
+#pragma unroll
+    for (int i = 0; i < M::Q; i++) f2[i].v.x = t[i] - SH * (float)M::w(i);
+  }
+  if (M::has_boundary(flb)) {
+    float t[M::Q];
+#pragma unroll
+    for (int i = 0; i < M::Q; i++) t[i] = f2[i].v.y + SH * (float)M::w(i);
+    M::pre_collision(t, flb, a);
+#pragma unroll
+    for (int i = 0; i < M::Q; i++) f2[i].v.y = t[i] - SH * (float)M::w(i);
+  }
+  const bool ca = M::collides(fla), cb = M::collides(flb);
+  if constexpr (LANES && M::identity_lanes) {
+    if (ca || cb) M::template collide_pair_lanes<SHIFTED>(f2, ca, cb, a);
+  } else if (ca || cb) {
+    // A pair where only one node collides (fluid next to a wall) parks the
+    // other node's values in thread-local memory across the collision; a
+    // volatile array keeps them out of the registers every pair would pay.
+    float keep_mem[M::Q];
+    volatile float* keep = keep_mem;
+    const bool mixed = ca != cb;
+    if (mixed) {
+#pragma unroll
+      for (int i = 0; i < M::Q; i++) keep[i] = ca ? f2[i].v.y : f2[i].v.x;
+    }
+    M::template collide_pair<SHIFTED>(f2, fla, flb, a);
+    if (mixed) {
+#pragma unroll
+      for (int i = 0; i < M::Q; i++) {
+        if (ca) f2[i].v.y = keep[i];
+        else f2[i].v.x = keep[i];
+      }
+    }
+  }
+}
+
 // Update and store two neighbouring nodes (x, x+1) of one row whose pulled
 // densities, as stored (shift not yet added), are v[i] = (node x, node x+1).
 // Models with a packed collision: boundary conditions per node, then one
@@ -1141,55 +1201,10 @@ __device__ __forceinline__ void pair_update_store(float2 (&v)[M::Q], flag_t fla,
                                                   unsigned node) {
   using P16 = Pack16<St>;
   if constexpr (M::packed && sizeof(R) == 4) {
-    // Values stay packed (node x, node x+1). A node with a boundary type has
-    // its lane taken out, updated by the scalar boundary code and put back;
-    // then one packed FP32x2 collision serves both nodes, so bulk and
-    // boundary pairs do not diverge in the collision.
-    // With shifted storage the packed values stay deviations g = f - w
-    // (the collision works on them directly); the scalar boundary code sees f.
-    constexpr float SH = St::shifted ? 1.0f : 0.0f;
     F2 f2[M::Q];
 #pragma unroll
     for (int i = 0; i < M::Q; i++) f2[i] = F2(v[i]);
-    if (M::has_boundary(fla)) {
-      float t[M::Q];
-#pragma unroll
-      for (int i = 0; i < M::Q; i++) t[i] = f2[i].v.x + SH * (float)M::w(i);
-      M::pre_collision(t, fla, a);
-#pragma unroll
-      for (int i = 0; i < M::Q; i++) f2[i].v.x = t[i] - SH * (float)M::w(i);
-    }
-    if (M::has_boundary(flb)) {
-      float t[M::Q];
-#pragma unroll
-      for (int i = 0; i < M::Q; i++) t[i] = f2[i].v.y + SH * (float)M::w(i);
-      M::pre_collision(t, flb, a);
-#pragma unroll
-      for (int i = 0; i < M::Q; i++) f2[i].v.y = t[i] - SH * (float)M::w(i);
-    }
-    const bool ca = M::collides(fla), cb = M::collides(flb);
-    if constexpr (LANES && M::identity_lanes) {
-      if (ca || cb) M::template collide_pair_lanes<St::shifted>(f2, ca, cb, a);
-    } else if (ca || cb) {
-      // A pair where only one node collides (fluid next to a wall) parks the
-      // other node's values in thread-local memory across the collision; a
-      // volatile array keeps them out of the registers every pair would pay.
-      float keep_mem[M::Q];
-      volatile float* keep = keep_mem;
-      const bool mixed = ca != cb;
-      if (mixed) {
-#pragma unroll
-        for (int i = 0; i < M::Q; i++) keep[i] = ca ? f2[i].v.y : f2[i].v.x;
-      }
-      M::template collide_pair<St::shifted>(f2, fla, flb, a);
-      if (mixed) {
-#pragma unroll
-        for (int i = 0; i < M::Q; i++) {
-          if (ca) f2[i].v.y = keep[i];
-          else f2[i].v.x = keep[i];
-        }
-      }
-    }
+    pair_update<M, St::shifted, LANES>(f2, fla, flb, a);
 #pragma unroll
     for (int i = 0; i < M::Q; i++) v[i] = f2[i].v;
   } else {

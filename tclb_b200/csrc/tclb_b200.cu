@@ -19,6 +19,7 @@
 #include <utility>
 
 #include "../../include/tclb_b200.h"
+#include "lbm_rows.cuh"
 #include "lbm_tma.cuh"
 
 using namespace tclb;
@@ -175,6 +176,9 @@ struct tclb_lattice {
   int lanes = 0;
   unsigned* count_dev = nullptr;  // device word for the count
   TmaMaps tma[2];
+  // plain iterations advanced per launch where there are that many left (1:
+  // one at a time)
+  int steps = 1;
   int* err_dev = nullptr;
   // failure-path test of the tile-staged kernel (tclb_set_fault_injection):
   // the tile whose copies are not issued (-1: none) and the wait bound
@@ -184,6 +188,7 @@ struct tclb_lattice {
 
 struct Impl {
   void (*iterate)(tclb_lattice*, bool, cudaStream_t);
+  void (*iterate_steps)(tclb_lattice*, cudaStream_t);  // L->steps plain iterations, from buf[cur] to buf[1 - cur]
   int (*flags_changed)(tclb_lattice*);  // after new node types: the kernel choices that depend on them
   void (*init)(tclb_lattice*, cudaStream_t);
   void (*quantity)(tclb_lattice*, int, int, const int*, double, void*, cudaStream_t);
@@ -224,11 +229,11 @@ inline bool tma_path(const tclb_lattice* L) {
 // kernel on the stream drains (the kernel itself waits for it with
 // griddepcontrol.wait); captured into CUDA graphs as a programmatic edge.
 template <class... KArgs, class... Args>
-void launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, cudaStream_t s, Args&&... args) {
+void launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
-  cfg.dynamicSmemBytes = 0;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -290,17 +295,46 @@ struct Launch {
         k_iterate_pair<M, R, St><<<grd, blk, 0, s>>>(a, P);
         return;
       }
-      if (glob) launch_pdl(k_iterate<M, R, St, true, PlaneAddr<T, M::Q>>, grid_of(L), dim3(L->bx, L->by), s, a, P);
-      else launch_pdl(k_iterate<M, R, St, false, PlaneAddr<T, M::Q>>, grid_of(L), dim3(L->bx, L->by), s, a, P);
+      if (glob) launch_pdl(k_iterate<M, R, St, true, PlaneAddr<T, M::Q>>, grid_of(L), dim3(L->bx, L->by), 0, s, a, P);
+      else launch_pdl(k_iterate<M, R, St, false, PlaneAddr<T, M::Q>>, grid_of(L), dim3(L->bx, L->by), 0, s, a, P);
     } else {
       const StrideAddr<T> P{static_cast<const T*>(src), static_cast<T*>(dst), L->stride};
-      if (glob) launch_pdl(k_iterate<M, R, St, true, StrideAddr<T>>, grid_of(L), dim3(L->bx, L->by), s, a, P);
-      else launch_pdl(k_iterate<M, R, St, false, StrideAddr<T>>, grid_of(L), dim3(L->bx, L->by), s, a, P);
+      if (glob) launch_pdl(k_iterate<M, R, St, true, StrideAddr<T>>, grid_of(L), dim3(L->bx, L->by), 0, s, a, P);
+      else launch_pdl(k_iterate<M, R, St, false, StrideAddr<T>>, grid_of(L), dim3(L->bx, L->by), 0, s, a, P);
     }
+  }
+  // Two iterations per launch (k_iterate_rows): two nodes per lane where rows
+  // of pairs line up (even nx, 32- and 16-bit storage), else one.
+  static constexpr bool rows_pair = M::DIM == 2 && sizeof(typename St::T) <= 4;
+  static constexpr bool rows_one = M::DIM == 2 && sizeof(typename St::T) >= 4;
+  template <bool PAIR>
+  static void launch_rows(tclb_lattice* L, cudaStream_t s) {
+    using E = typename St::T;
+    const auto a = make_args<M, R>(L, L->buf[L->cur], L->buf[1 - L->cur]);
+    PlaneAddr<E, M::Q> P;
+    for (int i = 0; i < M::Q; i++) {
+      P.s[i] = static_cast<const E*>(a.src) + (size_t)i * L->stride;
+      P.d[i] = static_cast<E*>(a.dst) + (size_t)i * L->stride;
+    }
+    constexpr int C = rows_columns<PAIR>(2);
+    const int strips = (L->nx + C - 1) / C, warps = strips * ((L->ny + ROWS_HEIGHT - 1) / ROWS_HEIGHT);
+    launch_pdl(k_iterate_rows<M, R, St, 2, PAIR>, dim3((warps + ROWS_WARPS - 1) / ROWS_WARPS), dim3(32 * ROWS_WARPS),
+               0, s, a, P, strips, ROWS_HEIGHT, warps);
+  }
+  static void iterate_steps(tclb_lattice* L, cudaStream_t s) {
+    if constexpr (rows_pair) {
+      if (L->nx % 2 == 0) return launch_rows<true>(L, s);
+    }
+    if constexpr (rows_one) launch_rows<false>(L, s);
+  }
+  static void prepare_steps(tclb_lattice* L) {
+    L->steps = 1;
+    if (M::DIM == 2 && L->N >= rows_min_nodes(sizeof(typename St::T)) && (rows_one || L->nx % 2 == 0)) L->steps = 2;
   }
   // Once at creation: the dynamic shared-memory limit and persistent grid of the
   // tile-staged kernel (resident blocks per SM x SMs, at most one per tile).
   static void prepare(tclb_lattice* L) {
+    prepare_steps(L);
     using T = typename St::T;
     if constexpr (sizeof(T) == 2) {
       if (!L->tma_ok) return;
@@ -384,8 +418,8 @@ struct Launch {
       for (size_t n = 0; n < N; n++) p[(size_t)q * stride + n] = St::from_double(in[(size_t)q * N + n], M::w(q));
   }
   static const Impl* get() {
-    static const Impl impl = {iterate,     flags_changed, init,    quantity, equilibrium, color,
-                              to_double,   from_double,   prepare, sizeof(R)};
+    static const Impl impl = {iterate, iterate_steps, flags_changed, init,    quantity, equilibrium, color,
+                              to_double, from_double, prepare, sizeof(R)};
     return &impl;
   }
 };
@@ -469,6 +503,20 @@ void drop_graphs(tclb_lattice* L) {
     }
 }
 
+// Enqueue up to n plain iterations in one launch; returns how many. 16-bit
+// storage takes several only where its single iterations take a two-node
+// kernel: the arithmetic, and so the result, does not depend on how a run is
+// cut into calls.
+int plain_steps(tclb_lattice* L, int n, cudaStream_t s) {
+  const bool packed = tma_path(L) || (L->use_pairs && L->nx % 64 == 0);
+  const bool set = L->tma_always || L->fault_tile >= 0 || L->wait_cycles != TMA_WAIT_CYCLES;  // staging asked for
+  const bool many = L->steps > 1 && n >= L->steps && (L->elem > 2 || (packed && !set));
+  if (many) L->impl->iterate_steps(L, s);
+  else L->impl->iterate(L, false, s);
+  L->cur = 1 - L->cur;
+  return many ? L->steps : 1;
+}
+
 // Capture GRAPH_CHUNK plain iterations starting from the current snapshot.
 int ensure_iter_graph(tclb_lattice* L, cudaStream_t s) {
   const int p = L->cur;
@@ -478,9 +526,7 @@ int ensure_iter_graph(tclb_lattice* L, cudaStream_t s) {
   cudaGraph_t g = nullptr;
   cudaError_t e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
-    for (int k = 0; k < GRAPH_CHUNK; k++) {
-      L->impl->iterate(L, false, cs);
-      L->cur = 1 - L->cur;
+    for (int k = 0; k < GRAPH_CHUNK; k += plain_steps(L, GRAPH_CHUNK - k, cs)) {
     }
     e = cudaStreamEndCapture(cs, &g);
   }
@@ -764,10 +810,10 @@ int tclb_iterate(tclb_h L, int niter, int iter_type, void* stream) {
   if (integ) last_glob = 0;
   bool globs = (iter_type & TCLB_ITER_GLOBS) != 0;
   int i = 0;
-  if (!globs && L->use_graphs) {
-    // plain iterations in graph replays of GRAPH_CHUNK (even: the snapshot
-    // parity is unchanged by a replay)
-    const int plain = niter - (last_glob ? 1 : 0);
+  const int plain = globs ? 0 : niter - (last_glob && niter > 0 ? 1 : 0);
+  if (L->use_graphs) {
+    // plain iterations in graph replays of GRAPH_CHUNK (an even number of launches, whether of one
+    // iteration or of two: the snapshot parity is unchanged by a replay)
     while (plain - i >= GRAPH_CHUNK) {
       int rc = ensure_iter_graph(L, s);
       if (rc) return rc;
@@ -775,6 +821,11 @@ int tclb_iterate(tclb_h L, int niter, int iter_type, void* stream) {
       i += GRAPH_CHUNK;
       L->iter += GRAPH_CHUNK;
     }
+  }
+  while (i < plain) {
+    const int n = plain_steps(L, plain - i, s);
+    i += n;
+    L->iter += n;
   }
   for (; i < niter; i++) {
     if (last_glob && i == niter - 1) {

@@ -1,0 +1,64 @@
+"""Two plain iterations per launch (2D lattices above a size): the same bits as
+one iteration per launch, whose kernels the other tests hold to the oracle."""
+import numpy as np
+import pytest
+
+from tclb_b200 import models as M
+from tclb_b200.lattice import Lattice
+
+from helpers import apply_params, random_flags
+
+pytestmark = pytest.mark.gpu
+
+TYPES = ["Wall", "Solid", "WVelocity", "EPressure", "NSymmetry", "EVelocity", "WPressure", "SVelocity"]
+PARAMS = [("setting", "Viscosity", 0.05), ("setting", "S3", 0.3), ("setting", "S4", 0.2),
+          ("setting", "GravitationX", 1e-6), ("setting", "GravitationY", -2e-6),
+          ("zone", "VelocityX", 0.02, 1), ("zone", "Pressure", 0.01, 1)]
+
+
+# widths that do and do not divide into strips (60 columns in pairs, 30 one per
+# lane), odd widths (one node per lane), heights below, at and off the 8 rows of
+# a segment; the narrowest lattice that wraps inside one strip
+@pytest.mark.parametrize("precision,storage,nx,ny", [
+    ("fp32", "same", 1500, 1000), ("fp32", "same", 1498, 1003), ("fp32", "same", 1449, 1051),
+    ("fp32", "same", 300000, 7), ("fp32", "same", 34, 45001), ("fp64", "same", 1024, 700), ("fp64", "same", 899, 801),
+    ("fp64", "same", 250000, 3), ("fp32", "fp16s", 1920, 1304), ("fp32", "bf16s", 256, 10001),
+    ("fp32", "fp16", 2560, 999)])
+def test_two_iterations_per_launch_match_single_ones(precision, storage, nx, ny):
+    fl = random_flags("d2q9", (1, ny, nx), TYPES, zones=2, seed=nx + ny, p_type=0.1)
+    rng = np.random.default_rng(ny)
+    real = np.float64 if precision == "fp64" else np.float32
+    rho = (1 + 0.01 * rng.standard_normal(nx * ny)).astype(real)
+    u = (0.02 * rng.standard_normal((nx * ny, 3))).astype(real)
+    out = []
+    for cuts in ([1] * 9, [9], [4, 5]):
+        g = Lattice("d2q9", nx, ny, precision=precision, storage=storage)
+        g.set_flags(fl)
+        apply_params(g, PARAMS)
+        g.init_equilibrium(rho, u)
+        for n in cuts:
+            g.Iterate(n, M.ITER_NORM)
+        g.sync()
+        assert g.iteration == 9
+        out.append(g.save())
+        g.close()
+    assert np.isfinite(out[0].view({"fp64": np.float64}.get(precision, np.float32))).all() or storage != "same"
+    assert out[0].tobytes() == out[1].tobytes()
+    assert out[0].tobytes() == out[2].tobytes()
+
+
+def test_graph_replays_of_two_iterations():
+    """More iterations than a graph holds, in one call and one by one."""
+    nx, ny = 1500, 1000
+    fl = random_flags("d2q9", (1, ny, nx), TYPES[:2], seed=5, p_type=0.05)
+    out = []
+    for cuts in ([1] * 75, [75]):
+        g = Lattice("d2q9", nx, ny, precision="fp32")
+        g.set_flags(fl)
+        apply_params(g, PARAMS)
+        g.Init()
+        for n in cuts:
+            g.Iterate(n, M.ITER_NORM | M.ITER_LASTGLOB if n == cuts[-1] and len(cuts) == 1 else M.ITER_NORM)
+        out.append(g.GetQuantity("U"))
+        g.close()
+    assert np.allclose(out[0], out[1], rtol=0, atol=1e-6)
