@@ -140,7 +140,7 @@ struct BL {
   }
   static void derive(BatchCase& C) {
     const Args<R, M::NSET> a = args_of<M, R>(C, nullptr, nullptr);
-    for (int i = 0; i < 4; i++) C.k[i] = (double)a.k[i];
+    for (int i = 0; i < NDERIVED; i++) C.k[i] = (double)a.k[i];
   }
   static int tma_grid(int sms) {
     if constexpr (pairs) {

@@ -59,7 +59,7 @@ struct BatchCase {
   int tma_rows;               // rows per staged tile; 0: the case is not staged
   const BatchTmaMaps* maps;   // with tma_rows > 0
   double s[BATCH_MAX_SET];
-  double k[4];  // per-case constants derived from s (Model::derived), computed on the host at admission
+  double k[NDERIVED];  // per-case constants derived from s (Model::derived), computed on the host at admission
 };
 
 struct BatchTile {
@@ -88,7 +88,7 @@ template <class R, int NSET>
 struct GroupArgs {
   typedef R real;
   const R (&s)[NSET];
-  const R (&k)[4];
+  const R (&k)[NDERIVED];
   const R* zone;
 };
 
@@ -127,7 +127,7 @@ __device__ __forceinline__ void case_args(const BatchCase& C, int parity, Args<R
 #pragma unroll
   for (int i = 0; i < M::NSET; i++) a.s[i] = (R)C.s[i];
 #pragma unroll
-  for (int i = 0; i < 4; i++) a.k[i] = (R)C.k[i];
+  for (int i = 0; i < NDERIVED; i++) a.k[i] = (R)C.k[i];
 }
 
 template <class M, class R, class St, bool G>

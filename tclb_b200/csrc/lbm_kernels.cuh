@@ -83,6 +83,7 @@ struct StoreBF16 {
 // ---------------------------------------------------------------------------
 // Kernel arguments
 // ---------------------------------------------------------------------------
+constexpr int NDERIVED = 5;
 template <class R, int NSET>
 struct Args {
   typedef R real;
@@ -94,7 +95,7 @@ struct Args {
   const R* zone;  // [zones][NZS] zonal settings
   double* glob;   // device Globals (FP64)
   R s[NSET];      // settings
-  R k[4];         // per-launch constants derived from the settings (Model::derived)
+  R k[NDERIVED];  // per-launch constants derived from the settings (Model::derived)
 };
 
 // AddTo<Global>(x) with TCLB's Objective rule: every AddTo of a SUM Global
@@ -121,7 +122,7 @@ struct D2Q9 {
   static constexpr int BATCH_MIN_BLOCKS = 6;  // one-tile batch kernel: <= 40 registers
   template <class R>
   __host__ __device__ static void derived(const R*, R* k) {
-    k[0] = k[1] = k[2] = k[3] = R(0);
+    for (int i = 0; i < NDERIVED; i++) k[i] = R(0);
   }
   __host__ __device__ static constexpr int ex(int i) { return (i == 1 || i == 5 || i == 8) ? 1 : ((i == 3 || i == 6 || i == 7) ? -1 : 0); }
   __host__ __device__ static constexpr int ey(int i) { return (i == 2 || i == 5 || i == 6) ? 1 : ((i == 4 || i == 7 || i == 8) ? -1 : 0); }
@@ -297,6 +298,7 @@ struct D2Q9 {
   // keeps its values (pair_update_store parks them).
   __device__ __forceinline__ static bool collides(flag_t fl) { return (fl & d2q9::MRT) != 0; }
   __device__ __forceinline__ static bool has_boundary(flag_t fl) { return (fl & d2q9::BOUNDARY) != 0; }
+  __device__ __forceinline__ static constexpr bool bounces(flag_t) { return false; }
   template <class R, class AR>
   __device__ __forceinline__ static void pre_collision(R (&f)[Q], flag_t fl, const AR& a) {
     boundaries(f, fl, a);
@@ -349,16 +351,24 @@ struct D3Q19 {
                        ZONE_SHIFT = d3q19::ZONE_SHIFT;
   static constexpr bool has_bulk = true;
   static constexpr bool packed = true;
-  // two-node kernel: 256 threads, <= 80 registers (3 blocks per SM), no spills
-  static constexpr int PAIR_THREADS = 256, PAIR_MIN_BLOCKS = 3;
+  // two-node kernel: blocks of 128 threads and 72 registers (28 warps per SM)
+  // measured faster, 52 bytes of spills included, than 256 threads and 80 (24
+  // warps) or 64 (32 warps): porous 384 x 192 x 192 FP16-shift 213.5 us against
+  // 258.8 and 234.9, 192^3 109.4 against 130.3 and 119.0
+  static constexpr int PAIR_THREADS = 128, PAIR_MIN_BLOCKS = 7;
   static constexpr int BATCH_MIN_BLOCKS = 5;  // one-tile batch kernel: <= 48 registers
-  // gamma1 = 1 - omega and gamma2 = 1 - 8(2 - omega)/(8 - omega), once per launch
+  // constants of trt(), once per launch: gamma1 = 1 - omega and
+  // gamma2 = 1 - 8(2 - omega)/(8 - omega) as gamma1, 1 - gamma1, gamma1 / 2,
+  // gamma2, gamma2 / 2
   template <class R>
   __host__ __device__ static void derived(const R* s, R* k) {
     const R omega = s[d3q19::S_omega];
     k[0] = R(1) - omega;
-    k[1] = R(1) - R(8) * (R(2) - omega) / (R(8) - omega);
-    k[2] = k[3] = R(0);
+    k[1] = omega;
+    k[2] = R(0.5) * k[0];
+    k[3] = R(1) - R(8) * (R(2) - omega) / (R(8) - omega);
+    k[4] = R(0.5) * k[3];
+    for (int i = 5; i < NDERIVED; i++) k[i] = R(0);
   }
   // directions: columns 4, 6, 8 of MRTMAT (d3q19/Dynamics.R:26-35)
   __host__ __device__ static constexpr int ex(int i) {
@@ -432,39 +442,35 @@ struct D3Q19 {
   //   rest:        rho/3 - (X+Y+Z)/3
   //   +-x axis:    rho/18 + X/6 - (Y+Z)/6     +-  Jx/6
   //   (sx,sy,0):   rho/36 + (X+Y)/12 + sx*sy*Jx*Jy/(4 rho)  +  (sx*Jx + sy*Jy)/12
-  // (and the same with the axes permuted).
-  // With EXACT_SUM the rest part is rho - 2 sum(e): the equilibrium then sums
-  // to rho up to the rounding of that sum, not to rho times the rounded
-  // weights' sum (1/3, 1/18, 1/36 are inexact in binary), which as a bias of
-  // ~1e-8 per iteration drifts the mass of a long FP32 run (5000 iterations:
-  // ~2e-4). Deviation storage (rho - 1 in place of rho) does not need it.
-  template <bool EXACT_SUM = false, class R>
-  __device__ __forceinline__ static void feq_parts(R rho, R irho, R jx, R jy, R jz, R& e0, R (&e)[9], R (&o)[9]) {
-    const R X = jx * jx * irho, Y = jy * jy * irho, Z = jz * jz * irho;
-    const R c18 = rho * R(1.0 / 18.0), c36 = rho * R(1.0 / 36.0);
-    if (!EXACT_SUM) e0 = (rho - X - Y - Z) * R(1.0 / 3.0);
-    e[0] = c18 + (X - Y - Z) * R(1.0 / 6.0);
-    e[1] = c18 + (Y - X - Z) * R(1.0 / 6.0);
-    e[2] = c18 + (Z - X - Y) * R(1.0 / 6.0);
-    const R xy = c36 + (X + Y) * R(1.0 / 12.0), pxy = R(0.25) * jx * jy * irho;
-    const R xz = c36 + (X + Z) * R(1.0 / 12.0), pxz = R(0.25) * jx * jz * irho;
-    const R yz = c36 + (Y + Z) * R(1.0 / 12.0), pyz = R(0.25) * jy * jz * irho;
-    e[3] = xy + pxy;  // 7 (1,1,0)
-    e[4] = xy - pxy;  // 8 (-1,1,0)
-    e[5] = xz + pxz;  // 11 (1,0,1)
-    e[6] = xz - pxz;  // 12 (-1,0,1)
-    e[7] = yz + pyz;  // 15 (0,1,1)
-    e[8] = yz - pyz;  // 16 (0,-1,1)
-    o[0] = jx * R(1.0 / 6.0);
-    o[1] = jy * R(1.0 / 6.0);
-    o[2] = jz * R(1.0 / 6.0);
-    o[3] = (jx + jy) * R(1.0 / 12.0);
-    o[4] = (jy - jx) * R(1.0 / 12.0);
-    o[5] = (jx + jz) * R(1.0 / 12.0);
-    o[6] = (jz - jx) * R(1.0 / 12.0);
-    o[7] = (jy + jz) * R(1.0 / 12.0);
-    o[8] = (jz - jy) * R(1.0 / 12.0);
-    if (EXACT_SUM) e0 = rho - R(2) * ((e[0] + e[1] + e[2]) + ((e[3] + e[4]) + (e[5] + e[6]) + (e[7] + e[8])));
+  // (and the same with the axes permuted). Given rho, X + Y + Z etc. as values
+  // of type V it is linear; even_parts and odd_parts are that linear map.
+  template <class V>
+  __device__ __forceinline__ static void even_parts(V rho, V X, V Y, V Z, V XY, V XZ, V YZ, V (&e)[9]) {
+    const V S = X + Y + Z;
+    const V c = V(1.0 / 18.0) * rho - V(1.0 / 6.0) * S, u = V(1.0 / 36.0) * rho + V(1.0 / 12.0) * S;
+    e[0] = V(1.0 / 3.0) * X + c;
+    e[1] = V(1.0 / 3.0) * Y + c;
+    e[2] = V(1.0 / 3.0) * Z + c;
+    const V xy = u - V(1.0 / 12.0) * Z, xz = u - V(1.0 / 12.0) * Y, yz = u - V(1.0 / 12.0) * X;
+    e[3] = xy + V(0.25) * XY;  // 7 (1,1,0)
+    e[4] = xy - V(0.25) * XY;  // 8 (-1,1,0)
+    e[5] = xz + V(0.25) * XZ;  // 11 (1,0,1)
+    e[6] = xz - V(0.25) * XZ;  // 12 (-1,0,1)
+    e[7] = yz + V(0.25) * YZ;  // 15 (0,1,1)
+    e[8] = yz - V(0.25) * YZ;  // 16 (0,-1,1)
+  }
+  template <class V>
+  __device__ __forceinline__ static void odd_parts(V jx, V jy, V jz, V (&o)[9]) {
+    const V x = V(1.0 / 12.0) * jx, y = V(1.0 / 12.0) * jy, z = V(1.0 / 12.0) * jz;
+    o[0] = x + x;
+    o[1] = y + y;
+    o[2] = z + z;
+    o[3] = x + y;
+    o[4] = y - x;
+    o[5] = x + z;
+    o[6] = z - x;
+    o[7] = y + z;
+    o[8] = z - y;
   }
 
   // CollisionMRT (:223-290). The d'Humieres rates of TCLB's d3q19 give every
@@ -474,18 +480,26 @@ struct D3Q19 {
   //   R <- S (R - Req(J)) + Req(J + rho F),  f = R . MRTMAT^-1
   // is therefore the same linear map as, in population space,
   //   f_i <- feq_i(J') + gamma1 (f - feq(J))_i^even + gamma2 (f - feq(J))_i^odd
-  // with even/odd parts taken over each pair (i, opposite i). It is evaluated
-  // that way here: pair sums and differences instead of two 19x19 transforms.
-  // The two-rate update for value type V (R, or F2 for two nodes); leaves
-  // rho and the forced momentum J' for the Globals. With DEV the values are
-  // deviations g = f - w: the sum of g is rho - 1, which enters the
-  // equilibrium's terms linear in rho (giving feq - w), while the quadratic
-  // terms and the force use the true density.
+  // with even/odd parts taken over each pair (i, opposite i), J' = J + rho F.
+  // The equilibrium is linear in rho, the products J_a J_b / rho and J, so
+  // feq(J') - gamma feq(J) is one evaluation of it at
+  //   (1 - gamma1) rho,  (1 - gamma1) J_a J_b / rho + [J'_a J'_b - J_a J_b] / rho,  J' - gamma2 J
+  // (the bracket is F_a J'_b + F_b J_a): about 150 operations, against 211
+  // with the equilibrium at J and at J' evaluated apart.
+  // For value type V (X1, or F2 for two nodes); leaves rho and J' for the
+  // Globals. The rest population is rho less the others: the mass is kept up
+  // to the rounding of that sum, not to that of the weights' sum (1/3, 1/18,
+  // 1/36 are inexact in binary), which as a bias of ~1e-8 per iteration would
+  // drift the mass of a long FP32 run (5000 iterations: ~2e-4). With DEV the
+  // values are deviations g = f - w: the sum of g is rho - 1, which enters the
+  // terms linear in rho (giving feq - w), while the quadratic terms and the
+  // force use the true density; the bias scales with rho - 1 and the rest
+  // population takes its own relaxation.
   // `lanes` (two-node form only) gives per-lane rates and force: a lane whose
   // node does not collide gets gamma1 = gamma2 = 1 and no force, which maps its
   // values onto themselves up to FP32 rounding (far below the 16-bit storage
   // the two-node form serves).
-  struct Lanes { F2 g1, g2, fx, fy, fz; };
+  struct Lanes { F2 g1, om, h1, g2, h2, fx, fy, fz; };
   template <bool DEV = false, class V, class AR>
   __device__ __forceinline__ static void trt(V (&f)[Q], const AR& a, V& rho, V& jx, V& jy, V& jz,
                                              const Lanes* lanes = nullptr) {
@@ -496,44 +510,51 @@ struct D3Q19 {
       d[p] = f[pair_a(p)] - f[pair_b(p)];
     }
     rho = f[0] + (s[0] + s[1] + s[2]) + ((s[3] + s[4]) + (s[5] + s[6]) + (s[7] + s[8]));
-    jx = d[0] + d[3] - d[4] + d[5] - d[6];
-    jy = d[1] + d[3] + d[4] + d[7] - d[8];
-    jz = d[2] + d[5] + d[6] + d[7] + d[8];
-    V g1, g2, fx, fy, fz;
+    const V mx = d[0] + d[3] - d[4] + d[5] - d[6];
+    const V my = d[1] + d[3] + d[4] + d[7] - d[8];
+    const V mz = d[2] + d[5] + d[6] + d[7] + d[8];
+    V g1 = V(a.k[0]), om = V(a.k[1]), h1 = V(a.k[2]), g2 = V(a.k[3]), h2 = V(a.k[4]);
+    V fx = V(a.s[d3q19::S_ForceX]), fy = V(a.s[d3q19::S_ForceY]), fz = V(a.s[d3q19::S_ForceZ]);
     if constexpr (std::is_same<V, F2>::value) {
       if (lanes) {
-        g1 = lanes->g1, g2 = lanes->g2, fx = lanes->fx, fy = lanes->fy, fz = lanes->fz;
-      } else {
-        g1 = V(a.k[0]), g2 = V(a.k[1]);
-        fx = V(a.s[d3q19::S_ForceX]), fy = V(a.s[d3q19::S_ForceY]), fz = V(a.s[d3q19::S_ForceZ]);
+        g1 = lanes->g1, om = lanes->om, h1 = lanes->h1, g2 = lanes->g2, h2 = lanes->h2;
+        fx = lanes->fx, fy = lanes->fy, fz = lanes->fz;
       }
-    } else {
-      g1 = V(a.k[0]), g2 = V(a.k[1]);
-      fx = V(a.s[d3q19::S_ForceX]), fy = V(a.s[d3q19::S_ForceY]), fz = V(a.s[d3q19::S_ForceZ]);
     }
     const V rho_t = DEV ? rho + V(1) : rho;  // true density
     const V irho = recip(rho_t);
-    V e0, e[9], o[9];
-    feq_parts<!DEV>(rho, irho, jx, jy, jz, e0, e, o);
-    jx += rho_t * fx;
-    jy += rho_t * fy;
-    jz += rho_t * fz;
-    V e0n, en[9], on[9];
-    feq_parts<!DEV>(rho, irho, jx, jy, jz, e0n, en, on);
-    f[0] = e0n + g1 * (f[0] - e0);
+    const V ux = mx * irho, uy = my * irho, uz = mz * irho;
+    jx = rho_t * fx + mx;
+    jy = rho_t * fy + my;
+    jz = rho_t * fz + mz;
+    const V X = om * V(ux * mx) + fx * (mx + jx), Y = om * V(uy * my) + fy * (my + jy),
+            Z = om * V(uz * mz) + fz * (mz + jz);
+    const V XY = fx * jy + (om * V(ux * my) + fy * mx), XZ = fx * jz + (om * V(ux * mz) + fz * mx),
+            YZ = fy * jz + (om * V(uy * mz) + fz * my);
+    const V r = om * rho;
+    V e[9], o[9];
+    even_parts(r, X, Y, Z, XY, XZ, YZ, e);
+    odd_parts(V(jx - g2 * mx), V(jy - g2 * my), V(jz - g2 * mz), o);
 #pragma unroll
     for (int p = 0; p < 9; p++) {
-      const V E = en[p] + g1 * (V(0.5) * s[p] - e[p]);
-      const V O = on[p] + g2 * (V(0.5) * d[p] - o[p]);
-      f[pair_a(p)] = E + O;
-      f[pair_b(p)] = E - O;
+      e[p] = h1 * s[p] + e[p];
+      o[p] = h2 * d[p] + o[p];
+      f[pair_a(p)] = e[p] + o[p];
+      f[pair_b(p)] = e[p] - o[p];
     }
+    if (DEV) f[0] = g1 * f[0] + V(1.0 / 3.0) * (r - (X + Y + Z));
+    else f[0] = rho - V(2) * ((e[0] + e[1] + e[2]) + ((e[3] + e[4]) + (e[5] + e[6]) + (e[7] + e[8])));
   }
 
   template <class R, bool G>
   __device__ __forceinline__ static void mrt(R (&f)[Q], flag_t fl, const Args<R, NSET>& a, R* g, const R* zs) {
-    R rho, jx, jy, jz;
-    trt(f, a, rho, jx, jy, jz);
+    X1<R> v[Q], xr, xx, xy, xz;
+#pragma unroll
+    for (int i = 0; i < Q; i++) v[i] = X1<R>(f[i]);
+    trt(v, a, xr, xx, xy, xz);
+#pragma unroll
+    for (int i = 0; i < Q; i++) f[i] = v[i].v;
+    const R rho = xr.v, jx = xx.v, jy = xy.v, jz = xz.v;
     if (G) {  // :266-289, with rho and J already divided by Mw = 19, 10 (C(R, Mw, eq="/="))
       const R rs = rho * R(1.0 / 19.0), px = jx * R(0.1), py = jy * R(0.1), pz = jz * R(0.1);
       const R ux = px / rs, uy = py / rs, uz = pz / rs;
@@ -620,6 +641,9 @@ struct D3Q19 {
   // its values; the rates are the same for every node).
   __device__ __forceinline__ static bool collides(flag_t fl) { return (fl & d3q19::COLLISION) == d3q19::MRT; }
   __device__ __forceinline__ static bool has_boundary(flag_t fl) { return (fl & d3q19::BOUNDARY) != 0; }
+  __device__ __forceinline__ static bool bounces(flag_t fl) {  // Solid or Wall
+    return (fl & d3q19::BOUNDARY) == d3q19::Wall || (fl & d3q19::BOUNDARY) == d3q19::Solid;
+  }
   template <class R, class AR>
   __device__ __forceinline__ static void pre_collision(R (&f)[Q], flag_t fl, const AR& a) {
     boundaries(f, fl, a);
@@ -637,20 +661,21 @@ struct D3Q19 {
   template <bool DEV, class AR>
   __device__ __forceinline__ static void collide_pair_lanes(F2 (&f)[Q], bool ca, bool cb, const AR& a) {
     F2 rho, jx, jy, jz;
-    const float g1 = (float)a.k[0], g2 = (float)a.k[1];
-    const float fx = (float)a.s[d3q19::S_ForceX], fy = (float)a.s[d3q19::S_ForceY], fz = (float)a.s[d3q19::S_ForceZ];
-    const Lanes L{F2(ca ? g1 : 1.0f, cb ? g1 : 1.0f), F2(ca ? g2 : 1.0f, cb ? g2 : 1.0f),
-                  F2(ca ? fx : 0.0f, cb ? fx : 0.0f), F2(ca ? fy : 0.0f, cb ? fy : 0.0f),
-                  F2(ca ? fz : 0.0f, cb ? fz : 0.0f)};
+    auto sel = [&](float on, float off) { return F2(ca ? on : off, cb ? on : off); };
+    const Lanes L{sel((float)a.k[0], 1.0f), sel((float)a.k[1], 0.0f), sel((float)a.k[2], 0.5f),
+                  sel((float)a.k[3], 1.0f), sel((float)a.k[4], 0.5f), sel((float)a.s[d3q19::S_ForceX], 0.0f),
+                  sel((float)a.s[d3q19::S_ForceY], 0.0f), sel((float)a.s[d3q19::S_ForceZ], 0.0f)};
     trt<DEV>(f, a, rho, jx, jy, jz, &L);
   }
 
   // SetEquilibrum (:212-217): f = Req(rho, J) . MRTMAT.inv
   template <class R>
   __device__ __forceinline__ static void equilibrium(R (&f)[Q], R rho, R jx, R jy, R jz) {
-    R e0, e[9], o[9];
-    feq_parts(rho, R(1) / rho, jx, jy, jz, e0, e, o);
-    f[0] = e0;
+    const R irho = R(1) / rho, X = jx * jx * irho, Y = jy * jy * irho, Z = jz * jz * irho;
+    R e[9], o[9];
+    even_parts(rho, X, Y, Z, jx * jy * irho, jx * jz * irho, jy * jz * irho, e);
+    odd_parts(jx, jy, jz, o);
+    f[0] = (rho - X - Y - Z) * R(1.0 / 3.0);
 #pragma unroll
     for (int p = 0; p < 9; p++) {
       f[pair_a(p)] = e[p] + o[p];
@@ -698,7 +723,7 @@ struct D3Q27C {
   __host__ __device__ static void derived(const R* s, R* k) {
     k[0] = R(1) / (R(3) * s[d3q27c::S_nu] + R(0.5));
     k[1] = R(1) / (R(3) * s[d3q27c::S_nubuffer] + R(0.5));
-    k[2] = k[3] = R(0);
+    for (int i = 2; i < NDERIVED; i++) k[i] = R(0);
   }
   // f<a><b><c>: index a + 3b + 9c, digit 0 -> 0, 1 -> +1, 2 -> -1
   __host__ __device__ static constexpr int dg(int v) { return v == 1 ? 1 : (v == 2 ? -1 : 0); }
@@ -865,6 +890,7 @@ struct D3Q27C {
   __device__ __forceinline__ static bool has_boundary(flag_t fl) {
     return (fl & (d3q27c::ADDITIONALS | d3q27c::BOUNDARY)) != 0;
   }
+  __device__ __forceinline__ static constexpr bool bounces(flag_t) { return false; }
   template <class R, class AR>
   __device__ __forceinline__ static void pre_collision(R (&f)[Q], flag_t fl, const AR& a) {
     if (fl & (d3q27c::ADDITIONALS | d3q27c::BOUNDARY)) {
@@ -1141,8 +1167,20 @@ __device__ __forceinline__ void pair_update(F2 (&f2)[M::Q], flag_t fla, flag_t f
   // boundary pairs do not diverge in the collision.
   // With shifted storage the packed values stay deviations g = f - w
   // (the collision works on them directly); the scalar boundary code sees f.
+  // Bounce-back exchanges opposite values, which have the same weight: on the
+  // packed deviations, without the weights. Only d3q19, the model of the porous
+  // media, has this path (M::bounces): in the d3q27 and d2q9 kernels the code
+  // alone costs 5% and 8% (code generation; Taylor-Green 256^3, 4096 x 1024).
   constexpr float SH = SHIFTED ? 1.0f : 0.0f;
-  if (M::has_boundary(fla)) {
+  if (M::bounces(fla)) {
+#pragma unroll
+    for (int i = 1; i < M::Q; i++)
+      if (M::opp(i) > i) {
+        const float t = f2[i].v.x;
+        f2[i].v.x = f2[M::opp(i)].v.x;
+        f2[M::opp(i)].v.x = t;
+      }
+  } else if (M::has_boundary(fla)) {
     float t[M::Q];
 #pragma unroll
     for (int i = 0; i < M::Q; i++) t[i] = f2[i].v.x + SH * (float)M::w(i);
@@ -1150,7 +1188,15 @@ __device__ __forceinline__ void pair_update(F2 (&f2)[M::Q], flag_t fla, flag_t f
 #pragma unroll
     for (int i = 0; i < M::Q; i++) f2[i].v.x = t[i] - SH * (float)M::w(i);
   }
-  if (M::has_boundary(flb)) {
+  if (M::bounces(flb)) {
+#pragma unroll
+    for (int i = 1; i < M::Q; i++)
+      if (M::opp(i) > i) {
+        const float t = f2[i].v.y;
+        f2[i].v.y = f2[M::opp(i)].v.y;
+        f2[M::opp(i)].v.y = t;
+      }
+  } else if (M::has_boundary(flb)) {
     float t[M::Q];
 #pragma unroll
     for (int i = 0; i < M::Q; i++) t[i] = f2[i].v.y + SH * (float)M::w(i);
