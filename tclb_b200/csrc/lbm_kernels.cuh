@@ -1020,36 +1020,60 @@ struct D3Q27C {
 };
 
 // ---------------------------------------------------------------------------
-// Globals: warp shuffle -> shared memory -> one FP64 atomic per Global per
-// block (replaces CudaAtomicAddReduceWarp / MaxReduceWarp, src/cross.hpp:163-181).
-// MAX Globals are non-negative here, so an integer max on the FP64 bits orders
-// them correctly.
+// The Globals of a block of the batch kernels: shared memory -> one warp per
+// Global -> one FP64 atomic per Global and block (replaces
+// CudaAtomicAddReduceWarp / MaxReduceWarp, src/cross.hpp:163-181). The threads
+// list their values in shared memory, a row of 256 per Global; a warp sums a
+// row in FP64, 8 values per lane, and shuffles the 32 partial sums. A Global
+// that is zero in all of a block, as the slices mostly are, costs one vote.
+// MAX Globals are non-negative, so an integer max on the FP64 bits orders them.
+// (The one-lattice kernel, k_iterate_globals, keeps sums over all its nodes.)
 // ---------------------------------------------------------------------------
+template <int NG, class R>
+constexpr int glob_rows() {  // rows in shared memory at once: 26 KB at most
+  return NG * (int)sizeof(R) <= 104 ? NG : 104 / (int)sizeof(R);
+}
+
+// One lane's part of the sum (or maximum) of a row of `threads` values.
+template <class R>
+__device__ __forceinline__ double glob_row(const R* row, int threads, int lane, bool sum) {
+  double v = 0.0;
+  for (int k = lane; k < threads; k += 32) {
+    const double u = (double)row[k];
+    v = sum ? v + u : (u > v ? u : v);
+  }
+  return v;
+}
+
+// The warp's lanes' parts of a Global -> *out.
+__device__ __forceinline__ void glob_flush(double v, int lane, bool sum, double* out) {
+  if (!__any_sync(0xffffffffu, v != 0.0)) return;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double u = __shfl_down_sync(0xffffffffu, v, o);
+    v = sum ? v + u : (u > v ? u : v);
+  }
+  if (lane > 0) return;
+  if (sum) atomicAdd(out, v);
+  else if (v > 0.0) atomicMax(reinterpret_cast<unsigned long long*>(out), (unsigned long long)__double_as_longlong(v));
+}
+
+// The Globals of one block (at most 256 threads, whole warps).
 template <int NG, int NSUM, class R>
 __device__ __forceinline__ void reduce_globals(const R (&g)[NG], double* out) {
-  __shared__ double sh[32][NG];
-  const int tid = threadIdx.x + blockDim.x * threadIdx.y;
+  constexpr int ROWS = glob_rows<NG, R>();
+  __shared__ R sh[ROWS][256];
+  const int tid = threadIdx.x + blockDim.x * threadIdx.y, threads = blockDim.x * blockDim.y;
   const int lane = tid & 31, warp = tid >> 5;
-  const int nwarps = (blockDim.x * blockDim.y + 31) >> 5;
 #pragma unroll
-  for (int i = 0; i < NG; i++) {
-    double v = (double)g[i];
+  for (int r0 = 0; r0 < NG; r0 += ROWS) {
+    if (r0 > 0) __syncthreads();  // the rows before have been read
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const double u = __shfl_down_sync(0xffffffffu, v, o);
-      v = i < NSUM ? v + u : (u > v ? u : v);
-    }
-    if (lane == 0) sh[warp][i] = v;
-  }
-  __syncthreads();
-  if (tid < NG) {
-    double v = sh[0][tid];
-    for (int w = 1; w < nwarps; w++) v = tid < NSUM ? v + sh[w][tid] : (sh[w][tid] > v ? sh[w][tid] : v);
-    if (tid < NSUM) {
-      if (v != 0.0) atomicAdd(out + tid, v);
-    } else if (v > 0.0) {
-      atomicMax(reinterpret_cast<unsigned long long*>(out + tid), (unsigned long long)__double_as_longlong(v));
-    }
+    for (int i = 0; i < ROWS; i++)
+      if (r0 + i < NG) sh[i][tid] = g[r0 + i];
+    __syncthreads();
+    for (int i = warp; i < ROWS && r0 + i < NG; i += threads >> 5)
+      glob_flush(glob_row(sh[i], threads, lane, r0 + i < NSUM), lane, r0 + i < NSUM, out + r0 + i);
   }
 }
 
@@ -1360,18 +1384,91 @@ __device__ __forceinline__ void pdl_wait_and_release() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-template <class M, class R, class St, bool G, class A>
+template <class M, class R, class St, class A>
 __global__ void __launch_bounds__(256) k_iterate(const Args<R, M::NSET> a, const A P) {
   pdl_wait_and_release();
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
   const int z = blockIdx.z;
-  const bool act = (x < a.nx) && (y < a.ny);
-  R g[G ? M::NG : 1];
+  R g[1];
+  if (x < a.nx && y < a.ny) node_update<M, R, St, false>(a, P, x, y, z, g);
+}
+
+// n / d for n < 2^31 by a multiplication: d <= 2^l, m = floor(2^(31+l) / d) + 1
+// < 2^32, and n m / 2^(31+l) exceeds n / d by less than 1 / d.
+struct FastDiv {
+  unsigned m, s, d;  // d == 1: m == 0
+  static FastDiv by(unsigned d) {
+    unsigned l = 0;
+    while ((1u << l) < d) l++;
+    return d == 1 ? FastDiv{0, 0, 1} : FastDiv{(unsigned)((1ull << (31 + l)) / d + 1), l - 1, d};
+  }
+  __device__ __forceinline__ unsigned div(unsigned n) const { return m ? __umulhi(n, m) >> s : n; }
+};
+struct FlatNodes {  // flat node index -> (x, y, z)
+  FastDiv row, plane;
+  unsigned nodes;
+  __device__ __forceinline__ void at(unsigned n, int& x, int& y, int& z) const {
+    z = (int)plane.div(n);
+    const unsigned r = n - (unsigned)z * plane.d;
+    y = (int)row.div(r);
+    x = (int)(r - (unsigned)y * row.d);
+  }
+};
+
+// An iteration that integrates the Globals: warps walk the flat node index
+// with a grid stride. A warp lists its nodes' values in shared memory, a row of
+// 32 per Global, and each lane adds up its part of one row in FP64 (all of it
+// for d3q19's 26 Globals, a third for d3q27's 10, an eighth for d2q9's 4): no
+// barrier and no shuffle until the warp's last nodes. Every warp shuffling
+// every Global through five FP64 steps, as before, was two thirds of the
+// instructions of a d3q19 Globals iteration (160^3 FP32: 196 M against 71 M of
+// a plain one).
+constexpr int GLOB_THREADS = 128;
+template <class M, class R, class St, class A>
+__global__ void __launch_bounds__(GLOB_THREADS) k_iterate_globals(const Args<R, M::NSET> a, const A P,
+                                                                  const FlatNodes F) {
+  constexpr int NG = M::NG, PARTS = 32 / NG;
+  __shared__ R sh[GLOB_THREADS / 32][NG * 33];
+  const int lane = threadIdx.x & 31, part = lane / NG, mine = lane - part * NG;
+  R* const row = sh[threadIdx.x >> 5];
+  const bool sum = mine < M::NSUM;
+  double acc = 0.0;
+  pdl_wait_and_release();
+  for (unsigned n0 = blockIdx.x * GLOB_THREADS + (threadIdx.x & ~31u); n0 < F.nodes; n0 += gridDim.x * GLOB_THREADS) {
+    R g[NG];
 #pragma unroll
-  for (int i = 0; i < (G ? M::NG : 1); i++) g[i] = 0;
-  if (act) node_update<M, R, St, G>(a, P, x, y, z, g);
-  if constexpr (G) reduce_globals<M::NG, M::NSUM, R>(g, a.glob);
+    for (int i = 0; i < NG; i++) g[i] = 0;
+    if (n0 + lane < F.nodes) {
+      int x, y, z;
+      F.at(n0 + lane, x, y, z);
+      node_update<M, R, St, true>(a, P, x, y, z, g);
+    }
+    __syncwarp();  // the rows before have been read
+#pragma unroll
+    for (int i = 0; i < NG; i++) row[i * 33 + lane] = g[i];
+    __syncwarp();
+    if (part < PARTS) {
+#pragma unroll
+      for (int k = 0; k < 32; k += PARTS)
+        if (k + part < 32) {
+          const double u = (double)row[mine * 33 + k + part];
+          acc = sum ? acc + u : (u > acc ? u : acc);
+        }
+    }
+  }
+  double v = acc;
+#pragma unroll
+  for (int p = 1; p < PARTS; p++) {
+    const double u = __shfl_sync(0xffffffffu, acc, mine + p * NG);
+    v = sum ? v + u : (u > v ? u : v);
+  }
+  if (lane >= NG) return;
+  if (sum) {
+    if (v != 0.0) atomicAdd(a.glob + lane, v);
+  } else if (v > 0.0) {
+    atomicMax(reinterpret_cast<unsigned long long*>(a.glob + lane), (unsigned long long)__double_as_longlong(v));
+  }
 }
 
 // BaseInit stage: equilibrium from settings, written to the current snapshot.

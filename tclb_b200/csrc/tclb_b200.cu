@@ -179,6 +179,7 @@ struct tclb_lattice {
   // plain iterations advanced per launch where there are that many left (1:
   // one at a time)
   int steps = 1;
+  int glob_grid = 0;  // blocks of a Globals iteration (set by the first)
   int* err_dev = nullptr;
   // failure-path test of the tile-staged kernel (tclb_set_fault_injection):
   // the tile whose copies are not issued (-1: none) and the wait bound
@@ -252,8 +253,24 @@ inline dim3 grid_of(const tclb_lattice* L) {
   return dim3((L->nx + L->bx - 1) / L->bx, (L->ny + L->by - 1) / L->by, L->nz);
 }
 
+FlatNodes flat_of(const tclb_lattice* L) {
+  return {FastDiv::by(L->nx), FastDiv::by((unsigned)L->nx * (unsigned)L->ny), (unsigned)L->N};
+}
+
 template <class M, class R, class St>
 struct Launch {
+  // As many blocks as the GPU holds at once, at most one thread per node.
+  template <class A>
+  static void launch_globals(tclb_lattice* L, cudaStream_t s, const Args<R, M::NSET>& a, const A& P) {
+    if (L->glob_grid == 0) {
+      int n = 0, sms = 0;
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_iterate_globals<M, R, St, A>, GLOB_THREADS, 0) != cudaSuccess ||
+          cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, L->device) != cudaSuccess)
+        return;  // the error is reported after the launches
+      L->glob_grid = (int)std::min<size_t>((L->N + GLOB_THREADS - 1) / GLOB_THREADS, (size_t)std::max(1, n) * sms);
+    }
+    launch_pdl(k_iterate_globals<M, R, St, A>, dim3(L->glob_grid), dim3(GLOB_THREADS), 0, s, a, P, flat_of(L));
+  }
   static void iterate(tclb_lattice* L, bool glob, cudaStream_t s) {
     const void* src = L->buf[L->cur];
     void* dst = L->buf[1 - L->cur];
@@ -295,12 +312,12 @@ struct Launch {
         k_iterate_pair<M, R, St><<<grd, blk, 0, s>>>(a, P);
         return;
       }
-      if (glob) launch_pdl(k_iterate<M, R, St, true, PlaneAddr<T, M::Q>>, grid_of(L), dim3(L->bx, L->by), 0, s, a, P);
-      else launch_pdl(k_iterate<M, R, St, false, PlaneAddr<T, M::Q>>, grid_of(L), dim3(L->bx, L->by), 0, s, a, P);
+      if (glob) launch_globals(L, s, a, P);
+      else launch_pdl(k_iterate<M, R, St, PlaneAddr<T, M::Q>>, grid_of(L), dim3(L->bx, L->by), 0, s, a, P);
     } else {
       const StrideAddr<T> P{static_cast<const T*>(src), static_cast<T*>(dst), L->stride};
-      if (glob) launch_pdl(k_iterate<M, R, St, true, StrideAddr<T>>, grid_of(L), dim3(L->bx, L->by), 0, s, a, P);
-      else launch_pdl(k_iterate<M, R, St, false, StrideAddr<T>>, grid_of(L), dim3(L->bx, L->by), 0, s, a, P);
+      if (glob) launch_globals(L, s, a, P);
+      else launch_pdl(k_iterate<M, R, St, StrideAddr<T>>, grid_of(L), dim3(L->bx, L->by), 0, s, a, P);
     }
   }
   // Two iterations per launch (k_iterate_rows): two nodes per lane where rows
