@@ -181,13 +181,14 @@ int tclb_sync(tclb_h h);
 /* Launch shape of the iteration kernel (bx multiple of 32, bx*by <= 256) and
    flags: TCLB_LAUNCH_GRAPHS replays runs of plain iterations from a captured
    CUDA graph (on by default); TCLB_LAUNCH_PAIRS lets 16-bit storage with
-   nx % 64 == 0 update two nodes per thread on plain iterations: 32-bit
+   an even nx update two nodes per thread on plain iterations: 32-bit
    accesses, and for d3q19 / d3q27_cumulant bulk nodes one packed FP32x2
    collision for both (on by default); TCLB_LAUNCH_TMA lets 16-bit storage
    stage tiles of whole rows in shared memory with TMA on plain iterations
    (on by default; it takes precedence over PAIRS) when nx is a multiple of 32
    up to 512 (tiles of whole rows, at most 512 nodes, the number of rows
-   dividing ny). bx, by shape the one-node kernel.
+   dividing ny). bx, by shape the one-node kernel of widths that are a
+   multiple of 32.
    A staging wait that runs out (about a second) is reported as TCLB_ERR_CUDA
    by the next tclb_sync or Globals-reading tclb_iterate. */
 #define TCLB_LAUNCH_GRAPHS 1

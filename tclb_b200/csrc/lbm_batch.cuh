@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(256, (G || sizeof(R) == 8) ? 1 : M::BATCH_MIN_
 // walking the rows with stride by; each warp covers 64 consecutive x of one
 // row. In the last tile of a row whose width is not a
 // multiple of 64 the lanes past the row only load (node_update_pair's
-// PARTIAL form). A case with odd nx has no node pairs: its tiles take the
+// PAIR_PARTIAL form). A case with odd nx has no node pairs: its tiles take the
 // one-node update, two nodes per thread.
 template <class M, class R, class St>
 __global__ void __launch_bounds__(M::PAIR_THREADS, M::PAIR_MIN_BLOCKS)
@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(M::PAIR_THREADS, M::PAIR_MIN_BLOCKS)
   }
   const int x = tile.x0 + 2 * threadIdx.x;
   for (int y = tile.y0 + threadIdx.y; y < y_end; y += blockDim.y)
-    node_update_pair<M, R, St, StrideAddr<T>, true>(a, P, x, y, z, threadIdx.x & 31);
+    node_update_pair<M, R, St, StrideAddr<T>, PAIR_PARTIAL>(a, P, x, y, z, threadIdx.x & 31);
 }
 
 // 16-bit storage, plain launches, cases whose rows fit one TMA box (see

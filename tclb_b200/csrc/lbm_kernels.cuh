@@ -1301,16 +1301,19 @@ __device__ __forceinline__ void pair_update_store(float2 (&v)[M::Q], flag_t fla,
   }
 }
 
-// PARTIAL: x may lie past the row (the last tile of a row whose width is not
-// a multiple of 64); such a lane loads the pair at x mod nx, which its
-// neighbours' shuffles need, and stores nothing.
-template <class M, class R, class St, class A, bool PARTIAL = false>
+// PAIR_ROW: the warp covers 64 nodes of one row. PAIR_PARTIAL: x may lie past
+// the row (the last tile of a row whose width is not a multiple of 64); such a
+// lane loads the pair at x mod nx, which its neighbours' shuffles need, and
+// stores nothing. PAIR_FLAT: the lanes hold consecutive pairs of the flat node
+// index, so a row may begin and end at any lane; the pairs at either end of a
+// row load their wrapped neighbour, and lanes with store = false only load.
+enum PairForm { PAIR_ROW, PAIR_PARTIAL, PAIR_FLAT };
+template <class M, class R, class St, class A, PairForm FORM = PAIR_ROW>
 __device__ __forceinline__ void node_update_pair(const Args<R, M::NSET>& a, const A& P, int x, int y, int z,
-                                                 int lane) {
+                                                 int lane, bool store = true) {
   using P16 = Pack16<St>;
   const unsigned nx = a.nx, ny = a.ny, nz = a.nz;
-  bool store = true;
-  if constexpr (PARTIAL) {
+  if constexpr (FORM == PAIR_PARTIAL) {
     if (x >= a.nx) {
       x = (unsigned)x % nx;
       store = false;
@@ -1322,6 +1325,8 @@ __device__ __forceinline__ void node_update_pair(const Args<R, M::NSET>& a, cons
   const unsigned oz_lo = z == 0 ? sxy * (nz - 1) : 0u - sxy, oz_hi = z + 1 == (int)nz ? sxy * (1u - nz) : sxy;
   const unsigned o_prev = x == 0 ? nx - 2 : 0u - 2u;       // pair (x-2, x-1), wrapped
   const unsigned o_next = x + 2 == (int)nx ? 2u - nx : 2u;  // pair (x+2, x+3), wrapped
+  const bool first = lane == 0 || (FORM == PAIR_FLAT && x == 0);             // the left pair is not the previous lane's
+  const bool last = lane == 31 || (FORM == PAIR_FLAT && x + 2 == (int)nx);  // nor the right one the next lane's
   const unsigned fl2 = __ldg(reinterpret_cast<const unsigned*>(a.flags + node));
   const flag_t fla = (flag_t)(fl2 & 0xffffu), flb = (flag_t)(fl2 >> 16);
   float2 v[M::Q];  // (node x, node x+1)
@@ -1336,15 +1341,15 @@ __device__ __forceinline__ void node_update_pair(const Args<R, M::NSET>& a, cons
       v[i] = P16::unpack(w);
     } else if (M::ex(i) > 0) {  // from x-1: (prev.hi, w.lo)
       unsigned prev = __shfl_up_sync(0xffffffffu, w, 1);
-      if (lane == 0) prev = __ldg(reinterpret_cast<const unsigned*>(base + (idx + o_prev)));
+      if (first) prev = __ldg(reinterpret_cast<const unsigned*>(base + (idx + o_prev)));
       v[i] = make_float2(P16::hi(prev), P16::lo(w));
     } else {  // from x+1: (w.hi, next.lo)
       unsigned next = __shfl_down_sync(0xffffffffu, w, 1);
-      if (lane == 31) next = __ldg(reinterpret_cast<const unsigned*>(base + (idx + o_next)));
+      if (last) next = __ldg(reinterpret_cast<const unsigned*>(base + (idx + o_next)));
       v[i] = make_float2(P16::hi(w), P16::lo(next));
     }
   }
-  if (!PARTIAL || store) pair_update_store<M, R, St, A, Args<R, M::NSET>, true>(v, fla, flb, a, P, node);
+  if (FORM == PAIR_ROW || store) pair_update_store<M, R, St, A, Args<R, M::NSET>, true>(v, fla, flb, a, P, node);
 }
 
 // Node pairs (2p, 2p+1) of the flat node index, p < npairs, of which exactly
@@ -1415,6 +1420,30 @@ struct FlatNodes {  // flat node index -> (x, y, z)
     x = (int)(r - (unsigned)y * row.d);
   }
 };
+
+// Widths that are not a multiple of 32: one thread per node of the flat index,
+// so that every warp is full and its stores start on a sector whatever nx is
+// (rows of 131 in blocks of 128 columns left half of every second block idle).
+template <class M, class R, class St, class A>
+__global__ void __launch_bounds__(256) k_iterate_flat(const Args<R, M::NSET> a, const A P, const FlatNodes F) {
+  const unsigned n = blockIdx.x * blockDim.x + threadIdx.x;
+  int x, y, z;
+  F.at(n, x, y, z);
+  pdl_wait_and_release();
+  R g[1];
+  if (n < F.nodes) node_update<M, R, St, false>(a, P, x, y, z, g);
+}
+
+// 16-bit storage, even widths that are not a multiple of 64: the two-node
+// update on consecutive pairs of the flat index.
+template <class M, class R, class St>
+__global__ void __launch_bounds__(M::PAIR_THREADS, M::PAIR_MIN_BLOCKS)
+    k_iterate_pair_flat(const Args<R, M::NSET> a, const PlaneAddr<typename St::T, M::Q> P, const FlatNodes F) {
+  const unsigned p = blockIdx.x * blockDim.x + threadIdx.x, pairs = F.nodes / 2;
+  int x, y, z;
+  F.at(2 * min(p, pairs - 1), x, y, z);
+  node_update_pair<M, R, St, PlaneAddr<typename St::T, M::Q>, PAIR_FLAT>(a, P, x, y, z, threadIdx.x & 31, p < pairs);
+}
 
 // An iteration that integrates the Globals: warps walk the flat node index
 // with a grid stride. A warp lists its nodes' values in shared memory, a row of

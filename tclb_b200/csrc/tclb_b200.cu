@@ -159,7 +159,7 @@ struct tclb_lattice {
   // settings travel as kernel parameters, so a settings change drops them.
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
   int use_graphs = 1;
-  int use_pairs = 1;  // 16-bit storage: two nodes per thread when nx % 64 == 0
+  int use_pairs = 1;  // 16-bit storage: two nodes per thread when nx is even
   // 16-bit storage: tile-staged TMA kernel (tma_rows rows per tile; tma[b]
   // describes snapshot b as the source), and its error word in the pool
   int use_tma = 1, tma_ok = 0, tma_rows = 0, tma_grid = 0;
@@ -271,6 +271,18 @@ struct Launch {
     }
     launch_pdl(k_iterate_globals<M, R, St, A>, dim3(L->glob_grid), dim3(GLOB_THREADS), 0, s, a, P, flat_of(L));
   }
+  // One node per thread.
+  template <class A>
+  static void launch_nodes(tclb_lattice* L, bool glob, cudaStream_t s, const Args<R, M::NSET>& a, const A& P) {
+    if (glob) return launch_globals(L, s, a, P);
+    if (L->nx % 32 == 0) {
+      launch_pdl(k_iterate<M, R, St, A>, grid_of(L), dim3(L->bx, L->by), 0, s, a, P);
+    } else {
+      const unsigned threads = 128;
+      launch_pdl(k_iterate_flat<M, R, St, A>, dim3((unsigned)((L->N + threads - 1) / threads)), dim3(threads), 0, s, a,
+                 P, flat_of(L));
+    }
+  }
   static void iterate(tclb_lattice* L, bool glob, cudaStream_t s) {
     const void* src = L->buf[L->cur];
     void* dst = L->buf[1 - L->cur];
@@ -312,12 +324,16 @@ struct Launch {
         k_iterate_pair<M, R, St><<<grd, blk, 0, s>>>(a, P);
         return;
       }
-      if (glob) launch_globals(L, s, a, P);
-      else launch_pdl(k_iterate<M, R, St, PlaneAddr<T, M::Q>>, grid_of(L), dim3(L->bx, L->by), 0, s, a, P);
+      if (L->use_pairs && !glob && L->nx % 2 == 0) {
+        const unsigned pairs = (unsigned)(L->N / 2);
+        k_iterate_pair_flat<M, R, St><<<(pairs + M::PAIR_THREADS - 1) / M::PAIR_THREADS, M::PAIR_THREADS, 0, s>>>(
+            a, P, flat_of(L));
+        return;
+      }
+      launch_nodes(L, glob, s, a, P);
     } else {
       const StrideAddr<T> P{static_cast<const T*>(src), static_cast<T*>(dst), L->stride};
-      if (glob) launch_globals(L, s, a, P);
-      else launch_pdl(k_iterate<M, R, St, StrideAddr<T>>, grid_of(L), dim3(L->bx, L->by), 0, s, a, P);
+      launch_nodes(L, glob, s, a, P);
     }
   }
   // Two iterations per launch (k_iterate_rows): two nodes per lane where rows
@@ -541,7 +557,7 @@ void drop_graphs(tclb_lattice* L) {
 // kernel: the arithmetic, and so the result, does not depend on how a run is
 // cut into calls.
 int plain_steps(tclb_lattice* L, int n, cudaStream_t s) {
-  const bool packed = tma_path(L) || (L->use_pairs && L->nx % 64 == 0);
+  const bool packed = tma_path(L) || (L->use_pairs && L->nx % 2 == 0);
   const bool set = L->tma_always || L->fault_tile >= 0 || L->wait_cycles != TMA_WAIT_CYCLES;  // staging asked for
   const bool many = L->steps > 1 && n >= L->steps && (L->elem > 2 || (packed && !set));
   if (many) L->impl->iterate_steps(L, s);
@@ -1218,7 +1234,7 @@ int tclb_get_launch(tclb_h L, int* bx, int* by, int* flags) {
   if (by) *by = L->by;
   if (flags) {
     const bool tma = tma_path(L);
-    const bool pairs = !tma && L->use_pairs && L->elem == 2 && L->nx % 64 == 0;
+    const bool pairs = !tma && L->use_pairs && L->elem == 2 && L->nx % 2 == 0;
     *flags = (L->use_graphs ? TCLB_LAUNCH_GRAPHS : 0) | (pairs ? TCLB_LAUNCH_PAIRS : 0) | (tma ? TCLB_LAUNCH_TMA : 0);
   }
   return TCLB_OK;
