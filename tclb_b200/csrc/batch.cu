@@ -50,6 +50,12 @@ struct LaunchTables {
   const BatchTmaTile* ttiles;  // tiles of the tile-staged kernel
   const int* nttiles;
   int* err;                    // set by a staging wait that ran out
+  const BatchRow* rows;        // strip segments of the cases that advance two iterations per launch
+  const int* nrows;
+  int nrows_grid;              // > 0: two iterations per launch, in this many blocks
+  int odd_grid;                // tiles of those cases: their single plain iteration
+  const BatchTile* odd_tiles;
+  const int* nodd;
 };
 
 struct BatchImpl {
@@ -70,10 +76,12 @@ struct BatchImpl {
   // the derived constants k of a case from its settings (host, in real_t)
   void (*derive)(BatchCase&);
   void (*clear)(BatchCase*, int n, int K, cudaStream_t);
+  void (*advance)(BatchCase*, int n, int K, bool two, cudaStream_t);
   void (*init)(const BatchCase&, const void* dst, cudaStream_t, int bx, int by);
   void (*quantity)(const BatchCase&, int parity, int q, int vec, double scale, void* out, cudaStream_t);
   int (*blocks_per_sm)(int threads);
-  const void* (*tile_kernel)(int which);  // 0 one-tile plain, 1 one-tile Globals, 2 pair
+  const void* (*tile_kernel)(int which);  // 0 one-tile plain, 1 one-tile Globals, 2 pair, 3 one-tile odd, 4 rows
+  bool (*takes_rows)(int nx);             // two iterations per launch possible for a case of this width
   int pair_threads;                        // block-size limit of the pair kernel; 0: no pair kernel
   bool group_staging;                      // staged cases must share their settings (packed collision)
   // smallest staged tile (nodes) of a case; cases with smaller tiles take the
@@ -108,17 +116,29 @@ template <class M, class R, class St>
 struct BL {
   // launch K-1 of a replay is every case's last iteration: the Globals variant
   static constexpr bool pairs = sizeof(typename St::T) == 2;  // 16-bit storage
+  static constexpr bool rows = M::DIM == 2 && !pairs;         // two iterations per launch
   static size_t tma_smem() { return tma_smem_bytes<M>(); }
   static void iterate(const LaunchTables& L, int k, int K, dim3 gp, dim3 ga, int tma_grid, const double* group,
                       int bx, int by, int form, bool plain_last, cudaStream_t s) {
     const dim3 b(bx, block_rows(bx, by, 256));
     const BatchCase* c = L.cases;
     const BatchTile* t = L.tiles;
+    const bool two = L.nrows_grid > 0;
+    if constexpr (rows) {
+      if (two) {
+        if (k % 2 == 1)
+          k_iterate_batch_rows<M, R, St, sizeof(R) == 4><<<L.nrows_grid, 32 * ROWS_WARPS, 0, s>>>(c, L.rows, L.nrows,
+                                                                                                k / 2, K);
+        if (k == K - 1)
+          k_iterate_batch_tile<M, R, St, ROLE_ODD><<<L.odd_grid, b, 0, s>>>(c, L.odd_tiles, L.nodd, k, K, two);
+      }
+    }
     if (k == K - 1) {  // every case's last iteration of the replay: the Globals variant, all tiles
       if (form == FORM_PERSISTENT) k_iterate_batch<M, R, St, true><<<gp, b, 0, s>>>(c, t, L.ntiles + 1, k, K);
-      else k_iterate_batch_tile<M, R, St, true><<<ga, b, 0, s>>>(c, t, L.ntiles + 1, k, K);
+      else k_iterate_batch_tile<M, R, St, ROLE_GLOBALS><<<ga, b, 0, s>>>(c, t, L.ntiles + 1, k, K, two);
       if (!plain_last) return;
     }
+    if (two && gp.x == 0) return;  // every case advances two iterations per launch
     if constexpr (pairs) {
       if (tma_grid > 0) {
         BatchCase G;  // the group's settings and derived constants
@@ -136,7 +156,7 @@ struct BL {
       }
     }
     if (form == FORM_PERSISTENT) k_iterate_batch<M, R, St, false><<<gp, b, 0, s>>>(c, t, L.ntiles, k, K);
-    else k_iterate_batch_tile<M, R, St, false><<<gp, b, 0, s>>>(c, t, L.ntiles, k, K);
+    else k_iterate_batch_tile<M, R, St, ROLE_PLAIN><<<gp, b, 0, s>>>(c, t, L.ntiles, k, K, two);
   }
   static void derive(BatchCase& C) {
     const Args<R, M::NSET> a = args_of<M, R>(C, nullptr, nullptr);
@@ -159,9 +179,17 @@ struct BL {
     if constexpr (pairs) {
       if (which == 2) return reinterpret_cast<const void*>(k_iterate_batch_pair<M, R, St>);
     }
-    if (which == 2) return nullptr;
-    return which ? reinterpret_cast<const void*>(k_iterate_batch_tile<M, R, St, true>)
-                 : reinterpret_cast<const void*>(k_iterate_batch_tile<M, R, St, false>);
+    if constexpr (rows) {
+      if (which == 3) return reinterpret_cast<const void*>(k_iterate_batch_tile<M, R, St, ROLE_ODD>);
+      if (which == 4) return reinterpret_cast<const void*>(k_iterate_batch_rows<M, R, St, sizeof(R) == 4>);
+    }
+    if (which >= 2) return nullptr;
+    return which ? reinterpret_cast<const void*>(k_iterate_batch_tile<M, R, St, ROLE_GLOBALS>)
+                 : reinterpret_cast<const void*>(k_iterate_batch_tile<M, R, St, ROLE_PLAIN>);
+  }
+  static bool takes_rows(int nx) { return rows && rows_case<R>(nx); }
+  static void advance(BatchCase* c, int n, int K, bool two, cudaStream_t s) {
+    k_batch_advance<R><<<(n + 127) / 128, 128, 0, s>>>(c, n, K, two);
   }
   // resident blocks per SM of the plain kernel at this block size
   static int blocks_per_sm(int threads) {
@@ -197,10 +225,12 @@ struct BL {
                                    tma_grid,
                                    derive,
                                    clear,
+                                   advance,
                                    init,
                                    quantity,
                                    blocks_per_sm,
                                    tile_kernel,
+                                   takes_rows,
                                    pairs ? M::PAIR_THREADS : 0,
                                    M::has_bulk,
                                    min_staged_nodes(),
@@ -267,11 +297,11 @@ CaseLayout case_layout(const BatchImpl* I, size_t elem, int nx, int ny, int nz) 
   return L;
 }
 
-// Per case (iterations done, left), then (error word of the staging waits, 0).
-__global__ void k_batch_status(const BatchCase* cases, int n, const int* err, int2* status) {
+// Per case (iterations done, left, launches done), then (error word of the staging waits).
+__global__ void k_batch_status(const BatchCase* cases, int n, const int* err, int4* status) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c < n) status[c] = make_int2(cases[c].counter, cases[c].remaining);
-  else if (c == n) status[n] = make_int2(*err, 0);
+  if (c < n) status[c] = make_int4(cases[c].counter, cases[c].remaining, cases[c].flips, 0);
+  else if (c == n) status[n] = make_int4(*err, 0, 0, 0);
 }
 
 }  // namespace
@@ -284,13 +314,19 @@ struct tclb_batch {
   cudaStream_t stream = nullptr;
   cudaMemPool_t pool = nullptr;
   BatchCase* d_cases = nullptr;
-  int2* d_status = nullptr;
-  int2* h_status = nullptr;  // pinned
-  int* d_ntiles = nullptr;   // [0] tiles of the cases not staged, [1] all tiles, [2] staged tiles
+  int4* d_status = nullptr;
+  int4* h_status = nullptr;  // pinned
+  int* d_ntiles = nullptr;   // [0] tiles of the cases not staged, [1] all tiles, [2] staged tiles, [3] odd tiles, [4] rows
   int* d_err = nullptr;      // staging wait ran out
   BatchTile* d_tiles = nullptr;
   BatchTmaTile* d_ttiles = nullptr;
-  size_t tiles_cap = 0, ttiles_cap = 0;
+  // two iterations per launch (k_iterate_batch_rows): the strip segments of
+  // the cases it takes and their tiles (for the single iterations)
+  BatchRow* d_rows = nullptr;
+  BatchTile* d_odd = nullptr;
+  size_t tiles_cap = 0, ttiles_cap = 0, rows_cap = 0, odd_cap = 0;
+  bool two = false;
+  int nrows = 0, nodd = 0;
   std::vector<BatchCase> cases;
   std::vector<size_t> bytes;
   std::vector<char> used_slot;
@@ -311,8 +347,9 @@ struct tclb_batch {
   cudaGraph_t graph_src = nullptr;          // kept: its nodes address the instantiated graph
   std::vector<cudaGraphNode_t> plain_nodes;  // one-block-per-tile plain launches
   std::vector<cudaGraphNode_t> glob_nodes;   // the Globals launch
-  int graph_grid[2] = {0, 0};                // their grids in the instantiated graph
-  int graph_key[8] = {-1, -1, -1, -1, -1, -1, -1, -1};
+  std::vector<cudaGraphNode_t> odd_nodes, rows_nodes;  // of the cases that advance two iterations per launch
+  int graph_grid[4] = {0, 0, 0, 0};          // their grids in the instantiated graph
+  int graph_key[9] = {-1, -1, -1, -1, -1, -1, -1, -1, -1};
   int paths = TCLB_LAUNCH_PAIRS | TCLB_LAUNCH_TMA | TCLB_BATCH_ADAPTIVE;  // tclb_batch_set_paths
 };
 
@@ -422,15 +459,41 @@ void update_staging(tclb_batch* B) {
   B->staging = on;
 }
 
+// Two iterations per launch for the cases k_iterate_batch_rows takes, where
+// they have nodes enough for it to be faster (the one-lattice rule).
+bool rows_case_of(const tclb_batch* B, size_t s) { return B->two && B->I->takes_rows(B->cases[s].nx); }
+void update_two(tclb_batch* B) {
+  size_t n = 0;
+  for (size_t s = 0; s < B->cases.size(); s++) {
+    const BatchCase& C = B->cases[s];
+    if (live(B, s) && B->I->takes_rows(C.nx)) n += (size_t)C.nx * C.ny;
+  }
+  B->two = B->user_grid == 0 && B->K >= 2 && n >= rows_min_nodes(B->elem);
+}
+
 int rebuild_tiles(tclb_batch* B) {
   update_staging(B);
-  std::vector<BatchTile> t;
+  update_two(B);
+  std::vector<BatchTile> t, odd;
   std::vector<BatchTmaTile> tt;
+  std::vector<BatchRow> rows;
   const int h = tile_height(B);
-  for (int pass = 0; pass < 2; pass++) {  // the cases not staged, then the staged ones
+  for (int pass = 0; pass < 2; pass++) {  // the cases not staged, then the staged ones and those of two iterations
     for (size_t s = 0; s < B->cases.size(); s++) {
       const BatchCase& C = B->cases[s];
-      if (!live(B, s) || staged(B, C) != (pass == 1)) continue;
+      const bool two = rows_case_of(B, s);
+      if (!live(B, s) || (staged(B, C) || two) != (pass == 1)) continue;
+      if (two) {
+        const int cols = B->elem == 8 ? rows_columns<false>(2) : rows_columns<true>(2);
+        for (int y = 0; y < C.ny; y += ROWS_HEIGHT)
+          for (int x = 0; x * cols < C.nx; x++) rows.push_back({(int)s, x, y});
+        for (int y = 0; y < C.ny; y += h)
+          for (int x = 0; x < C.nx; x += B->bx) {
+            t.push_back({(int)s, x, y, 0, h});
+            odd.push_back({(int)s, x, y, 0, h});
+          }
+        continue;
+      }
       for (int z = 0; z < C.nz; z++)
         for (int y = 0; y < C.ny; y += h)
           for (int x = 0; x < C.nx; x += B->bx) t.push_back({(int)s, x, y, z, h});
@@ -442,8 +505,15 @@ int rebuild_tiles(tclb_batch* B) {
   }
   B->tile_h = h;
   int rc;
-  if ((rc = reserve(B, B->d_tiles, B->tiles_cap, t.size())) || (rc = reserve(B, B->d_ttiles, B->ttiles_cap, tt.size())))
+  if ((rc = reserve(B, B->d_tiles, B->tiles_cap, t.size())) || (rc = reserve(B, B->d_ttiles, B->ttiles_cap, tt.size())) ||
+      (rc = reserve(B, B->d_rows, B->rows_cap, rows.size())) || (rc = reserve(B, B->d_odd, B->odd_cap, odd.size())))
     return rc;
+  B->nrows = (int)rows.size();
+  B->nodd = (int)odd.size();
+  if (!rows.empty()) {
+    BCK(cudaMemcpyAsync(B->d_rows, rows.data(), rows.size() * sizeof(BatchRow), cudaMemcpyHostToDevice, B->stream));
+    BCK(cudaMemcpyAsync(B->d_odd, odd.data(), odd.size() * sizeof(BatchTile), cudaMemcpyHostToDevice, B->stream));
+  }
   B->ntiles = (int)t.size();
   B->nttiles = (int)tt.size();
   if (!t.empty())
@@ -451,12 +521,14 @@ int rebuild_tiles(tclb_batch* B) {
   if (!tt.empty())
     BCK(cudaMemcpyAsync(B->d_ttiles, tt.data(), tt.size() * sizeof(BatchTmaTile), cudaMemcpyHostToDevice,
                         B->stream));
-  const int n[3] = {B->nplain, B->ntiles, B->nttiles};
+  const int n[5] = {B->nplain, B->ntiles, B->nttiles, B->nodd, B->nrows};
   BCK(cudaMemcpyAsync(B->d_ntiles, n, sizeof(n), cudaMemcpyHostToDevice, B->stream));
   BCK(cudaStreamSynchronize(B->stream));  // the host vectors die here
   B->tiles_dirty = false;
   return TCLB_OK;
 }
+
+int rows_grid(const tclb_batch* B) { return std::max(1, (B->nrows + ROWS_WARPS - 1) / ROWS_WARPS); }
 
 // One block per tile: the grid of the plain launches is the count of tiles
 // of the cases not staged, that of the Globals launch the count of all tiles.
@@ -464,10 +536,11 @@ int rebuild_tiles(tclb_batch* B) {
 // new grids in place (no recapture).
 int update_graph_grid(tclb_batch* B) {
   if (B->user_grid != 0) return TCLB_OK;
-  const int grid[2] = {std::max(1, B->nplain), std::max(1, B->ntiles)};
-  for (int w = 0; w < 2; w++) {
+  const int grid[4] = {std::max(1, B->nplain), std::max(1, B->ntiles), std::max(1, B->nodd), rows_grid(B)};
+  const std::vector<cudaGraphNode_t>* nodes[4] = {&B->plain_nodes, &B->glob_nodes, &B->odd_nodes, &B->rows_nodes};
+  for (int w = 0; w < 4; w++) {
     if (grid[w] == B->graph_grid[w]) continue;
-    for (cudaGraphNode_t node : (w ? B->glob_nodes : B->plain_nodes)) {
+    for (cudaGraphNode_t node : *nodes[w]) {
       cudaKernelNodeParams p;
       BCK(cudaGraphKernelNodeGetParams(node, &p));
       p.gridDim = dim3(grid[w]);
@@ -483,8 +556,10 @@ int ensure_graph(tclb_batch* B) {
   // the staged group's settings are captured as kernel parameters
   const int group_hash = (int)std::hash<std::string>()(
       std::string(reinterpret_cast<const char*>(B->group.data()), B->group.size() * sizeof(double)));
-  const int key[8] = {B->bx, B->by, B->K, (int)B->cases.size(), B->user_grid, B->paths, has_tma, group_hash};
-  if (B->graph && std::equal(key, key + 8, B->graph_key)) return update_graph_grid(B);
+  // with two iterations per launch: whether cases of one remain
+  const int forms = B->two ? (B->nplain > 0 ? 2 : 1) : 0;
+  const int key[9] = {B->bx, B->by, B->K, (int)B->cases.size(), B->user_grid, B->paths, has_tma, group_hash, forms};
+  if (B->graph && std::equal(key, key + 9, B->graph_key)) return update_graph_grid(B);
   if (B->graph) {
     cudaGraphExecDestroy(B->graph);
     B->graph = nullptr;
@@ -495,6 +570,8 @@ int ensure_graph(tclb_batch* B) {
   }
   B->plain_nodes.clear();
   B->glob_nodes.clear();
+  B->odd_nodes.clear();
+  B->rows_nodes.clear();
   const int threads = B->bx * block_rows(B->bx, B->by, 256);
   int per_sm = B->I->blocks_per_sm(threads);
   if (per_sm < 1) per_sm = std::max(1, 2048 / threads);
@@ -504,17 +581,18 @@ int ensure_graph(tclb_batch* B) {
   B->grid_blocks = per_tile ? std::max(1, B->nplain) : (B->user_grid > 0 ? B->user_grid : B->sms * per_sm);
   const int grid_all = per_tile ? std::max(1, B->ntiles) : B->grid_blocks;
   const int form = !per_tile ? FORM_PERSISTENT : (pair_form(B) ? FORM_PAIR : FORM_TILE);
-  const LaunchTables L = {B->d_cases, B->d_tiles, B->d_ntiles, B->d_ttiles, B->d_ntiles + 2, B->d_err};
+  const LaunchTables L = {B->d_cases, B->d_tiles, B->d_ntiles, B->d_ttiles, B->d_ntiles + 2, B->d_err, B->d_rows,
+                          B->d_ntiles + 4, B->two ? rows_grid(B) : 0, std::max(1, B->nodd), B->d_odd, B->d_ntiles + 3};
   cudaGraph_t g;
   BCK(cudaStreamBeginCapture(B->stream, cudaStreamCaptureModeThreadLocal));
   const int n = (int)B->cases.size();
   B->I->clear(B->d_cases, n, B->K, B->stream);
   for (int k = 0; k < B->K; k++)
-    B->I->iterate(L, k, B->K, dim3(B->grid_blocks), dim3(grid_all), has_tma ? B->tma_grid : 0,
+    B->I->iterate(L, k, B->K, dim3(forms == 1 ? 0 : B->grid_blocks), dim3(grid_all), has_tma ? B->tma_grid : 0,
                   B->group.empty() ? nullptr : B->group.data(), B->bx, B->by, form,
                   (B->paths & TCLB_BATCH_GLOBALS_AT_END) != 0, B->stream);
   if (n > 0) {
-    k_batch_advance<<<(n + 127) / 128, 128, 0, B->stream>>>(B->d_cases, n, B->K);
+    B->I->advance(B->d_cases, n, B->K, B->two, B->stream);
     k_batch_status<<<(n + 128) / 128, 128, 0, B->stream>>>(B->d_cases, n, B->d_err, B->d_status);
   }
   cudaError_t e = cudaStreamEndCapture(B->stream, &g);
@@ -533,6 +611,8 @@ int ensure_graph(tclb_batch* B) {
     const void* f0 = B->I->tile_kernel(0);
     const void* f1 = B->I->tile_kernel(1);
     const void* f2 = B->I->tile_kernel(2);
+    const void* f3 = B->I->tile_kernel(3);
+    const void* f4 = B->I->tile_kernel(4);
     for (cudaGraphNode_t node : nodes) {
       cudaGraphNodeType type;
       BCK(cudaGraphNodeGetType(node, &type));
@@ -541,11 +621,15 @@ int ensure_graph(tclb_batch* B) {
       BCK(cudaGraphKernelNodeGetParams(node, &p));
       if (p.func == f0 || (f2 && p.func == f2)) B->plain_nodes.push_back(node);
       else if (p.func == f1) B->glob_nodes.push_back(node);
+      else if (f3 && p.func == f3) B->odd_nodes.push_back(node);
+      else if (f4 && p.func == f4) B->rows_nodes.push_back(node);
     }
   }
   B->graph_grid[0] = B->grid_blocks;
   B->graph_grid[1] = grid_all;
-  std::copy(key, key + 8, B->graph_key);
+  B->graph_grid[2] = L.odd_grid;
+  B->graph_grid[3] = rows_grid(B);
+  std::copy(key, key + 9, B->graph_key);
   return TCLB_OK;
 }
 
@@ -572,7 +656,7 @@ int fill_case(tclb_batch* B, int slot, char* p, const CaseLayout& L, const Model
   C.nx = nx;
   C.ny = ny;
   C.nz = nz;
-  C.counter = 0;
+  C.counter = C.flips = 0;
   C.remaining = niter;
   C.active = 1;
   C.glob_end = (B->paths & TCLB_BATCH_GLOBALS_AT_END) ? 1 : 0;
@@ -657,14 +741,14 @@ int tclb_batch_create(tclb_batch_h* out, int model, int precision, int storage, 
   }
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&B->stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaMalloc((void**)&B->d_cases, sizeof(BatchCase) * max_cases);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&B->d_status, sizeof(int2) * (max_cases + 1));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&B->d_ntiles, 3 * sizeof(int));
+  if (e == cudaSuccess) e = cudaMalloc((void**)&B->d_status, sizeof(int4) * (max_cases + 1));
+  if (e == cudaSuccess) e = cudaMalloc((void**)&B->d_ntiles, 5 * sizeof(int));
   if (e == cudaSuccess) e = cudaMalloc((void**)&B->d_err, sizeof(int));
   if (e == cudaSuccess) e = cudaMemset(B->d_err, 0, sizeof(int));
-  if (e == cudaSuccess) e = cudaMallocHost((void**)&B->h_status, sizeof(int2) * (max_cases + 1));
-  if (e == cudaSuccess) std::memset(B->h_status, 0, sizeof(int2) * (max_cases + 1));
+  if (e == cudaSuccess) e = cudaMallocHost((void**)&B->h_status, sizeof(int4) * (max_cases + 1));
+  if (e == cudaSuccess) std::memset(B->h_status, 0, sizeof(int4) * (max_cases + 1));
   if (e == cudaSuccess) e = cudaMemset(B->d_cases, 0, sizeof(BatchCase) * max_cases);
-  if (e == cudaSuccess) e = cudaMemset(B->d_ntiles, 0, 3 * sizeof(int));
+  if (e == cudaSuccess) e = cudaMemset(B->d_ntiles, 0, 5 * sizeof(int));
   if (e != cudaSuccess) {
     tclb_batch_destroy(B);
     return bfail(TCLB_ERR_CUDA, std::string("batch create: ") + cudaGetErrorString(e));
@@ -682,6 +766,8 @@ int tclb_batch_destroy(tclb_batch_h B) {
     if (B->used_slot[s]) cudaFreeAsync(B->cases[s].buf[0], B->stream);
   if (B->d_tiles) cudaFreeAsync(B->d_tiles, B->stream);
   if (B->d_ttiles) cudaFreeAsync(B->d_ttiles, B->stream);
+  if (B->d_rows) cudaFreeAsync(B->d_rows, B->stream);
+  if (B->d_odd) cudaFreeAsync(B->d_odd, B->stream);
   if (B->stream) cudaStreamSynchronize(B->stream);
   if (B->d_cases) cudaFree(B->d_cases);
   if (B->d_status) cudaFree(B->d_status);
@@ -728,7 +814,7 @@ int tclb_batch_add_case(tclb_batch_h B, int nx, int ny, int nz, const uint16_t* 
   B->bytes[slot] = L.total;
   B->used_slot[slot] = 1;
   B->used += L.total;
-  B->h_status[slot] = make_int2(0, niter);
+  B->h_status[slot] = make_int4(0, niter, 0, 0);
   B->tiles_dirty = true;
   *case_id = slot;
   return TCLB_OK;
@@ -843,7 +929,7 @@ int tclb_batch_step(tclb_batch_h B) {
   if ((rc = ensure_graph(B))) return rc;
   BCK(cudaGraphLaunch(B->graph, B->stream));
   B->status_n = (int)B->cases.size();
-  BCK(cudaMemcpyAsync(B->h_status, B->d_status, sizeof(int2) * (B->status_n + 1), cudaMemcpyDeviceToHost,
+  BCK(cudaMemcpyAsync(B->h_status, B->d_status, sizeof(int4) * (B->status_n + 1), cudaMemcpyDeviceToHost,
                       B->stream));
   return TCLB_OK;
 }
@@ -903,7 +989,7 @@ int tclb_batch_get_quantity(tclb_batch_h B, int id, int q, void* out, double sca
   const size_t bytes = (size_t)C.nx * C.ny * C.nz * (vec ? 3 : 1) * B->I->real_size;
   void* tmp = nullptr;
   BCK(cudaMallocFromPoolAsync(&tmp, bytes, B->pool, B->stream));
-  const int parity = B->h_status[id].x & 1;
+  const int parity = B->h_status[id].z & 1;
   B->I->quantity(C, parity, q, vec, scale, tmp, B->stream);
   BCK(cudaGetLastError());
   BCK(cudaMemcpyAsync(out, tmp, bytes, cudaMemcpyDeviceToHost, B->stream));

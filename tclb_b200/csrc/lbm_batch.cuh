@@ -27,12 +27,19 @@
 // compute Globals in this replay: every replay, or with glob_end only the
 // finishing one; the others take the plain kernels at K-1 too), and the plain
 // launches carry no Globals code (the register count of the one-lattice
-// kernel, not of both paths). Its A/B parity at launch k is
-// (counter + k - (K - d)) & 1. The counters advance only in k_batch_advance
-// at the end of a replay, so a CUDA graph of K launches + advance can be
-// replayed while cases come and go.
+// kernel, not of both paths). A case counts its launches (`flips`), and its
+// A/B parity at launch k is (flips + k - (K - d)) & 1. The counters advance
+// only in k_batch_advance at the end of a replay, so a CUDA graph of K
+// launches + advance can be replayed while cases come and go.
+//
+// 2D batches large enough to be bound by HBM advance the cases that
+// k_iterate_rows takes two iterations per launch (k_iterate_batch_rows): of
+// the p plain iterations a case has in a replay, p / 2 launches of two (the
+// last ones of K / 2), then one launch of one where p is odd, then the
+// Globals launch.
 #pragma once
 #include "lbm_kernels.cuh"
+#include "lbm_rows.cuh"
 #include "lbm_tma.cuh"
 
 namespace tclb {
@@ -53,6 +60,7 @@ struct BatchCase {
   size_t stride;
   int nx, ny, nz;
   int counter;    // iterations done
+  int flips;      // launches done (each writes the other snapshot)
   int remaining;  // iterations left
   int active;
   int glob_end;               // 1: Globals only in the replay where the case finishes
@@ -105,9 +113,41 @@ __device__ __forceinline__ bool case_runs(const BatchCase& C, int k, int K, bool
   const int remaining = C.remaining;
   const int d = remaining < K ? remaining : K;
   const int first = K - d;
-  parity = (C.counter + (k - first)) & 1;
+  parity = (C.flips + (k - first)) & 1;
   const bool on = C.active && d > 0 && k >= first;
   return k == K - 1 ? on && G == case_globals(C, K) : on && !G;
+}
+
+// The launches of a case in a replay of K that advances it two iterations per
+// launch: `twos` of them, a single one if `odd`, the Globals one if `glob`.
+struct CaseTwos {
+  int twos;
+  bool odd, glob;
+};
+__device__ __forceinline__ CaseTwos case_twos(const BatchCase& C, int K) {
+  const int d = C.remaining < K ? C.remaining : K;
+  if (!C.active || d <= 0) return {0, false, false};
+  const bool glob = case_globals(C, K);
+  const int plain = d - (glob ? 1 : 0);
+  return {plain / 2, (plain & 1) != 0, glob};
+}
+// Whether k_iterate_batch_rows takes a case of width nx: pairs need an even
+// width, FP64 has one node per lane.
+template <class R>
+__host__ __device__ constexpr bool rows_case(int nx) { return sizeof(R) == 8 || nx % 2 == 0; }
+
+// What a launch of the one-node kernels runs: launch k of K of the cases that
+// advance one iteration per launch (`two`: not those of k_iterate_batch_rows),
+// the single plain iteration of the others, or the Globals iteration of all.
+enum BatchRole { ROLE_PLAIN, ROLE_ODD, ROLE_GLOBALS };
+template <class R, BatchRole ROLE>
+__device__ __forceinline__ bool case_on(const BatchCase& C, int k, int K, bool two, int& parity) {
+  if (two && rows_case<R>(C.nx)) {
+    const CaseTwos t = case_twos(C, K);
+    parity = (C.flips + t.twos + (ROLE == ROLE_GLOBALS && t.odd ? 1 : 0)) & 1;
+    return ROLE == ROLE_ODD ? t.odd : (ROLE == ROLE_GLOBALS && t.glob);
+  }
+  return ROLE != ROLE_ODD && case_runs(C, k, K, ROLE == ROLE_GLOBALS, parity);
 }
 
 // The node-update arguments of case C at the given parity (the derived
@@ -176,16 +216,16 @@ __global__ void __launch_bounds__(256) k_iterate_batch(const BatchCase* __restri
 
 // The arguments of tile t at launch k of a replay of K; false if the block
 // has nothing to do (past the live tiles, or the case idle at this launch).
-template <class M, class R, bool G>
+template <class M, class R, BatchRole ROLE>
 __device__ __forceinline__ bool batch_tile_args(const BatchCase* __restrict__ cases,
                                                 const BatchTile* __restrict__ tiles, const int* __restrict__ ntiles_p,
-                                                int k, int K, BatchTile& tile, Args<R, M::NSET>& a) {
+                                                int k, int K, bool two, BatchTile& tile, Args<R, M::NSET>& a) {
   const int t = blockIdx.x;
   if (t >= *ntiles_p) return false;
   tile = tiles[t];
   const BatchCase& C = cases[tile.slot];
   int parity;
-  if (!case_runs(C, k, K, G, parity)) return false;
+  if (!case_on<R, ROLE>(C, k, K, two, parity)) return false;
   case_args<M, R>(C, parity, a);
   return true;
 }
@@ -193,13 +233,14 @@ __device__ __forceinline__ bool batch_tile_args(const BatchCase* __restrict__ ca
 // One block per tile (grid = live tiles): blocks are independent, as in the
 // one-lattice kernel. A block of bx x by threads walks the tile's h rows with
 // stride by, so its descriptor reads are spread over h / by nodes per thread.
-template <class M, class R, class St, bool G>
-__global__ void __launch_bounds__(256, (G || sizeof(R) == 8) ? 1 : M::BATCH_MIN_BLOCKS)
+template <class M, class R, class St, BatchRole ROLE>
+__global__ void __launch_bounds__(256, (ROLE == ROLE_GLOBALS || sizeof(R) == 8) ? 1 : M::BATCH_MIN_BLOCKS)
     k_iterate_batch_tile(const BatchCase* __restrict__ cases, const BatchTile* __restrict__ tiles,
-                         const int* __restrict__ ntiles_p, int k, int K) {
+                         const int* __restrict__ ntiles_p, int k, int K, bool two) {
+  constexpr bool G = ROLE == ROLE_GLOBALS;
   BatchTile tile;
   Args<R, M::NSET> a;
-  if (!batch_tile_args<M, R, G>(cases, tiles, ntiles_p, k, K, tile, a)) return;
+  if (!batch_tile_args<M, R, ROLE>(cases, tiles, ntiles_p, k, K, two, tile, a)) return;
   const int x = tile.x0 + threadIdx.x, z = tile.z;
   const int y_end = min(tile.y0 + tile.h, a.ny);
   using T = typename St::T;
@@ -231,7 +272,7 @@ __global__ void __launch_bounds__(M::PAIR_THREADS, M::PAIR_MIN_BLOCKS)
                          const int* __restrict__ ntiles_p, int k, int K) {
   BatchTile tile;
   Args<R, M::NSET> a;
-  if (!batch_tile_args<M, R, false>(cases, tiles, ntiles_p, k, K, tile, a)) return;
+  if (!batch_tile_args<M, R, ROLE_PLAIN>(cases, tiles, ntiles_p, k, K, false, tile, a)) return;
   using T = typename St::T;
   const StrideAddr<T> P{static_cast<const T*>(a.src), static_cast<T*>(a.dst), a.stride};
   const int z = tile.z;
@@ -417,12 +458,42 @@ __global__ void __launch_bounds__(TMA_THREADS, 2)
   }
 }
 
+// One warp per strip segment of k_iterate_rows, over the cases of a batch:
+// launch j of the K / 2 launches of two iterations in a replay of K.
+struct BatchRow {
+  int slot, strip, y0;
+};
+template <class M, class R, class St, bool PAIR>
+__global__ void __launch_bounds__(ROWS_WARPS * 32, sizeof(R) == 8 ? 4 : 5)  // the case's settings: no spills at 5
+    k_iterate_batch_rows(const BatchCase* __restrict__ cases, const BatchRow* __restrict__ rows,
+                         const int* __restrict__ nrows_p, int j, int K) {
+  __shared__ RowRing<St, M::Q, PAIR> ring[ROWS_WARPS];
+  const int wid = threadIdx.x >> 5, w = blockIdx.x * ROWS_WARPS + wid;
+  if (w >= *nrows_p) return;
+  const BatchRow row = rows[w];
+  const BatchCase& C = cases[row.slot];
+  const int n = case_twos(C, K).twos, first = K / 2 - n;
+  if (j < first) return;
+  Args<R, M::NSET> a;
+  case_args<M, R>(C, (C.flips + (j - first)) & 1, a);
+  using T = typename St::T;
+  rows_walk<M, R, St, 2, PAIR>(a, StrideAddr<T>{static_cast<const T*>(a.src), static_cast<T*>(a.dst), a.stride},
+                               row.strip, row.y0, ring[wid]);
+}
+
 // End of a replay: counters and remaining iterations of every active case.
-__global__ void k_batch_advance(BatchCase* cases, int ncases, int K) {
+template <class R>
+__global__ void k_batch_advance(BatchCase* cases, int ncases, int K, bool two) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= ncases || !cases[c].active) return;
   const int r = cases[c].remaining;
   const int d = r < K ? r : K;
+  if (two && rows_case<R>(cases[c].nx)) {
+    const CaseTwos t = case_twos(cases[c], K);
+    cases[c].flips += t.twos + (t.odd ? 1 : 0) + (t.glob ? 1 : 0);
+  } else {
+    cases[c].flips += d;
+  }
   cases[c].counter += d;
   cases[c].remaining = r - d;
 }

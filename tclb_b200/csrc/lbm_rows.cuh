@@ -86,36 +86,52 @@ __device__ __forceinline__ void copy_ahead(unsigned smem, const void* p) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem), "l"(p), "n"(BYTES) : "memory");
 }
 
-template <class M, class R, class St, int T, bool PAIR>
-__global__ void __launch_bounds__(ROWS_WARPS * 32, sizeof(R) == 8 ? 4 : 6)
-    k_iterate_rows(const Args<R, M::NSET> a, const PlaneAddr<typename St::T, M::Q> P, int strips, int H, int nwarps) {
+// The staged rows of a warp: population i of row y from row y - e_y, and the
+// node types (the word that holds them).
+template <class St, int Q, bool PAIR>
+struct RowRing {
+  typename std::conditional_t<PAIR, RowPair<St>, RowOne<St>>::Raw f[ROWS_AHEAD + 1][Q][32];
+  unsigned types[ROWS_AHEAD + 1][32];
+};
+
+template <class M, class R, class St, bool PAIR, class Raw, class AR>
+__device__ __forceinline__ void rows_update(Raw (&f)[M::Q], unsigned fl, const AR& a) {
+  if constexpr (PAIR) {
+    using Row = RowPair<St>;
+    F2 v[M::Q];
+#pragma unroll
+    for (int i = 0; i < M::Q; i++) v[i] = Row::get(f[i]);
+    pair_update<M, St::shifted, false>(v, (flag_t)(fl & 0xffffu), (flag_t)(fl >> 16), a);
+#pragma unroll
+    for (int i = 0; i < M::Q; i++) f[i] = Row::put(v[i]);
+  } else {
+    M::template run<R, false>(f, (flag_t)fl, a, (R*)nullptr);
+  }
+}
+
+// One warp's work: output rows y0 .. of one strip, T iterations from the
+// source planes of P to its destination planes.
+template <class M, class R, class St, int T, bool PAIR, class A, class AR>
+__device__ __forceinline__ void rows_walk(const AR& a, const A& P, int strip, int y0, RowRing<St, M::Q, PAIR>& ring) {
   static_assert(M::DIM == 2 && T >= 2, "2D models, two iterations or more");
   static_assert(PAIR || !St::shifted, "one node per lane: 32- and 64-bit storage");
   using Row = std::conditional_t<PAIR, RowPair<St>, RowOne<St>>;
   using Raw = typename Row::Raw;
-  using F = std::conditional_t<PAIR, unsigned, flag_t>;  // a lane's node types
   constexpr int Q = M::Q, LOST = rows_lost<PAIR>(T), PER = PAIR ? 2 : 1;
-  const int w = blockIdx.x * ROWS_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31;
   const int nx = a.nx, ny = a.ny;
-  const int seg = w / strips;
-  const int x0 = (w - seg * strips) * rows_columns<PAIR>(T) - LOST + PER * lane;  // not wrapped
+  const int x0 = strip * rows_columns<PAIR>(T) - LOST + PER * lane;  // not wrapped
   const bool mine = PER * lane >= LOST && PER * lane < 32 * PER - LOST && x0 < nx;
   int x = x0 % nx;
   if (x < 0) x += nx;
   const int xm = x == 0 ? nx - 1 : x - 1, xp = x + 1 == nx ? 0 : x + 1;  // one node per lane
-  const int y0 = seg * H, rows = min(H, ny - y0) + 2 * (T - 1);
+  const int rows = min(ROWS_HEIGHT, ny - y0) + 2 * (T - 1);
   int y = (y0 - (T - 1)) % ny;
   if (y < 0) y += ny;
   unsigned o = (unsigned)nx * (unsigned)y0 + (unsigned)x;  // node of the first output row
-  pdl_wait_and_release();
-  if (w >= nwarps) return;
 
-  // Source rows staged ahead in shared memory: population i of row y from row
-  // y - e_y, and the node types (the word that holds them). Copies that pass
-  // by the registers leave the warp free to run on its other values.
-  __shared__ __align__(16) Raw ring[ROWS_WARPS][ROWS_AHEAD + 1][Q][32];
-  __shared__ unsigned fring[ROWS_WARPS][ROWS_AHEAD + 1][32];
-  const int wid = threadIdx.x >> 5;
+  // Copies ahead that pass by the registers leave the warp free to run on its
+  // other values.
   auto pull = [&](int slot, int y) {
     const unsigned r0 = (unsigned)nx * (unsigned)y;
     const unsigned rm = (unsigned)nx * (unsigned)(y == 0 ? ny - 1 : y - 1);
@@ -124,29 +140,16 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32, sizeof(R) == 8 ? 4 : 6)
     for (int i = 0; i < Q; i++) {
       const unsigned r = M::ey(i) == 0 ? r0 : (M::ey(i) > 0 ? rm : rp);
       const int c = PAIR || M::ex(i) == 0 ? x : (M::ex(i) > 0 ? xm : xp);
-      copy_ahead<sizeof(Raw)>((unsigned)__cvta_generic_to_shared(&ring[wid][slot][i][lane]), P.src(i) + (r + (unsigned)c));
+      copy_ahead<sizeof(Raw)>((unsigned)__cvta_generic_to_shared(&ring.f[slot][i][lane]), P.src(i) + (r + (unsigned)c));
     }
-    copy_ahead<4>((unsigned)__cvta_generic_to_shared(&fring[wid][slot][lane]),
+    copy_ahead<4>((unsigned)__cvta_generic_to_shared(&ring.types[slot][lane]),
                   a.flags + ((r0 + (unsigned)x) & ~1u));
   };
   auto shift = [&](int i, Raw v) -> Raw {
     return M::ex(i) == 0 ? v : (M::ex(i) > 0 ? Row::from_left(v) : Row::from_right(v));
   };
-  auto update = [&](Raw(&f)[Q], F fl) {
-    if constexpr (PAIR) {
-      F2 v[Q];
-#pragma unroll
-      for (int i = 0; i < Q; i++) v[i] = Row::get(f[i]);
-      pair_update<M, St::shifted, false>(v, (flag_t)(fl & 0xffffu), (flag_t)(fl >> 16), a);
-#pragma unroll
-      for (int i = 0; i < Q; i++) f[i] = Row::put(v[i]);
-    } else {
-      M::template run<R, false>(f, fl, a, (R*)nullptr);
-    }
-  };
-
   Raw e0[T - 1][Q], e1[T - 1][Q], e2[T - 1][Q];  // rows kept between the stages (entries not used vanish)
-  F fl[T];
+  unsigned fl[T];  // node types of the rows in flight, the lane's one or two
 #pragma unroll
   for (int k = 0; k < T - 1; k++) {
 #pragma unroll
@@ -171,15 +174,15 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32, sizeof(R) == 8 ? 4 : 6)
     __syncwarp();  // every lane's copies of this row; and all have read the row that is overwritten next
     Raw f[Q];
 #pragma unroll
-    for (int i = 0; i < Q; i++) f[i] = PAIR ? shift(i, ring[wid][slot][i][lane]) : ring[wid][slot][i][lane];
+    for (int i = 0; i < Q; i++) f[i] = PAIR ? shift(i, ring.f[slot][i][lane]) : ring.f[slot][i][lane];
 #pragma unroll
     for (int k = T - 1; k > 0; k--) fl[k] = fl[k - 1];
-    if constexpr (PAIR) fl[0] = fring[wid][slot][lane];
-    else fl[0] = (flag_t)(fring[wid][slot][lane] >> (((unsigned)nx * (unsigned)yr + (unsigned)x) & 1u ? 16 : 0));
+    if constexpr (PAIR) fl[0] = ring.types[slot][lane];
+    else fl[0] = (flag_t)(ring.types[slot][lane] >> (((unsigned)nx * (unsigned)yr + (unsigned)x) & 1u ? 16 : 0));
     yr = yr + 1 == ny ? 0 : yr + 1;
     slot = slot == ROWS_AHEAD ? 0 : slot + 1;
     stage();
-    update(f, fl[0]);
+    rows_update<M, R, St, PAIR>(f, fl[0], a);
 #pragma unroll
     for (int k = 0; k < T - 1; k++) {
       // f: row r after stage k+1; pull for stage k+2 at row r-1
@@ -199,7 +202,7 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32, sizeof(R) == 8 ? 4 : 6)
         }
       }
       // rows before the stage's first are not complete: not updated, not stored
-      if (j >= 2 * (k + 1)) update(g, fl[k + 1]);
+      if (j >= 2 * (k + 1)) rows_update<M, R, St, PAIR>(g, fl[k + 1], a);
 #pragma unroll
       for (int i = 0; i < Q; i++) f[i] = g[i];
     }
@@ -211,6 +214,17 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32, sizeof(R) == 8 ? 4 : 6)
       o += (unsigned)nx;
     }
   }
+}
+
+template <class M, class R, class St, int T, bool PAIR>
+__global__ void __launch_bounds__(ROWS_WARPS * 32, sizeof(R) == 8 ? 4 : 6)
+    k_iterate_rows(const Args<R, M::NSET> a, const PlaneAddr<typename St::T, M::Q> P, int strips, int nwarps) {
+  __shared__ RowRing<St, M::Q, PAIR> ring[ROWS_WARPS];
+  const int wid = threadIdx.x >> 5, w = blockIdx.x * ROWS_WARPS + wid;
+  pdl_wait_and_release();
+  if (w >= nwarps) return;
+  const int seg = w / strips;
+  rows_walk<M, R, St, T, PAIR>(a, P, w - seg * strips, seg * ROWS_HEIGHT, ring[wid]);
 }
 
 }  // namespace tclb

@@ -352,7 +352,7 @@ struct Launch {
     constexpr int C = rows_columns<PAIR>(2);
     const int strips = (L->nx + C - 1) / C, warps = strips * ((L->ny + ROWS_HEIGHT - 1) / ROWS_HEIGHT);
     launch_pdl(k_iterate_rows<M, R, St, 2, PAIR>, dim3((warps + ROWS_WARPS - 1) / ROWS_WARPS), dim3(32 * ROWS_WARPS),
-               0, s, a, P, strips, ROWS_HEIGHT, warps);
+               0, s, a, P, strips, warps);
   }
   static void iterate_steps(tclb_lattice* L, cudaStream_t s) {
     if constexpr (rows_pair) {

@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 
 from tclb_b200 import models as M
+from tclb_b200.batch import Batch, CaseSpec
 from tclb_b200.lattice import Lattice
 
 from helpers import apply_params, random_flags
@@ -62,3 +63,37 @@ def test_graph_replays_of_two_iterations():
         out.append(g.GetQuantity("U"))
         g.close()
     assert np.allclose(out[0], out[1], rtol=0, atol=1e-6)
+
+
+# iterations per replay even, odd and one; iteration counts that end anywhere in
+# a replay; a case of odd width (one iteration per launch among the others in
+# FP32); Globals in every replay and at the end
+@pytest.mark.parametrize("at_end", [True, False])
+@pytest.mark.parametrize("K", [1, 5, 8])
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_batch_of_two_iterations_per_launch(precision, K, at_end):
+    shapes = [(1000, 1600), (45, 301), (64, 128), (257, 640)]
+    iters = [13, 10, 3, 16]
+    b = Batch("d2q9", precision, budget_bytes=8 << 30)
+    b.set_paths(globals_at_end=at_end)
+    b.set_launch(64, 16, K)
+    specs = [CaseSpec(random_flags("d2q9", (1,) + sh, TYPES[:2] + ["WVelocity"], zones=2, seed=k, p_type=0.05),
+                      {"Viscosity": 0.05, "GravitationX": 1e-6}, {0: {"VelocityX": 0.02}, 1: {"VelocityX": 0.01}}, n)
+             for k, (sh, n) in enumerate(zip(shapes, iters))]
+    ids = [b.add_case(s) for s in specs]
+    b.run_to_completion()
+    for cid, s in zip(ids, specs):
+        assert b.poll(cid) == (s.niter, 0)
+        ny, nx = s.flags.shape[1:]
+        g = Lattice("d2q9", nx, ny, precision=precision)
+        g.set_flags(s.flags)
+        apply_params(g, [("setting", k, v) for k, v in s.settings.items()])
+        for z, d in s.zone_settings.items():
+            g.set_zone_setting("VelocityX", d["VelocityX"], z)
+        g.Init()
+        g.Iterate(s.niter, M.ITER_NORM | M.ITER_LASTGLOB)
+        assert np.array_equal(b.quantity(cid, "U"), g.GetQuantity("U")), (nx, ny)
+        # FP64 sums in another order
+        assert np.allclose(b.globals(cid), g.globals, rtol=1e-6 if precision == "fp32" else 1e-9, atol=1e-9)
+        g.close()
+    b.close()
