@@ -19,6 +19,7 @@
 
 #include "../../include/tclb_b200.h"
 #include "lbm_batch.cuh"
+#include "read_back.h"
 
 using namespace tclb;
 
@@ -350,6 +351,7 @@ struct tclb_batch {
   std::vector<cudaGraphNode_t> odd_nodes, rows_nodes;  // of the cases that advance two iterations per launch
   int graph_grid[4] = {0, 0, 0, 0};          // their grids in the instantiated graph
   int graph_key[9] = {-1, -1, -1, -1, -1, -1, -1, -1, -1};
+  ReadBack read_back;
   int paths = TCLB_LAUNCH_PAIRS | TCLB_LAUNCH_TMA | TCLB_BATCH_ADAPTIVE;  // tclb_batch_set_paths
 };
 
@@ -992,9 +994,9 @@ int tclb_batch_get_quantity(tclb_batch_h B, int id, int q, void* out, double sca
   const int parity = B->h_status[id].z & 1;
   B->I->quantity(C, parity, q, vec, scale, tmp, B->stream);
   BCK(cudaGetLastError());
-  BCK(cudaMemcpyAsync(out, tmp, bytes, cudaMemcpyDeviceToHost, B->stream));
+  const cudaError_t e = B->read_back.copy(out, tmp, bytes, B->stream, B->device);
   BCK(cudaFreeAsync(tmp, B->stream));
-  BCK(cudaStreamSynchronize(B->stream));
+  BCK(e);
   return TCLB_OK;
 }
 

@@ -21,6 +21,7 @@
 #include "../../include/tclb_b200.h"
 #include "lbm_rows.cuh"
 #include "lbm_tma.cuh"
+#include "read_back.h"
 
 using namespace tclb;
 
@@ -175,6 +176,8 @@ struct tclb_lattice {
   // 64.5-65.1k; without such pairs, Taylor-Green, parking is 1.3% faster)
   int lanes = 0;
   unsigned* count_dev = nullptr;  // device word for the count
+  char* scalars = nullptr;  // pinned words that small results arrive in
+  ReadBack read_back;
   TmaMaps tma[2];
   // plain iterations advanced per launch where there are that many left (1:
   // one at a time)
@@ -600,14 +603,19 @@ int set_setting_rec(tclb_lattice* L, int i, double v, int depth) {
 }
 
 // Lattice::calcGlobals (src/Lattice.cu.Rt:1299-1315): device Globals -> host
-// accumulators, then clear the device copy.
+// accumulators, then clear the device copy. The error word of the staged
+// kernel follows the Globals in the pool, so one copy and one wait read both.
 int calc_globals(tclb_lattice* L, cudaStream_t s) {
-  std::vector<double> tab(L->T->nglobals);
-  TCLB_CK(cudaMemcpyAsync(tab.data(), L->glob_dev, tab.size() * sizeof(double), cudaMemcpyDeviceToHost, s));
+  const int n = L->T->nglobals;
+  const size_t err_at = (size_t)(reinterpret_cast<char*>(L->err_dev) - reinterpret_cast<char*>(L->glob_dev));
+  TCLB_CK(cudaMemcpyAsync(L->scalars, L->glob_dev, err_at + sizeof(int), cudaMemcpyDeviceToHost, s));
+  TCLB_CK(cudaMemsetAsync(L->glob_dev, 0, n * sizeof(double), s));
   TCLB_CK(cudaStreamSynchronize(s));
-  for (size_t i = 0; i < tab.size(); i++) L->globals[i] += tab[i];
-  TCLB_CK(cudaMemsetAsync(L->glob_dev, 0, tab.size() * sizeof(double), s));
-  return check_device_error(L, s);
+  const double* tab = reinterpret_cast<const double*>(L->scalars);
+  for (int i = 0; i < n; i++) L->globals[i] += tab[i];
+  int e = 0;
+  std::memcpy(&e, L->scalars + err_at, sizeof(int));
+  return e ? check_device_error(L, s) : TCLB_OK;
 }
 
 #define CHECK_H(h) \
@@ -698,7 +706,9 @@ int tclb_create(tclb_h* out, int model, int nx, int ny, int nz, int precision, i
   L->glob_dev = reinterpret_cast<double*>(L->pool + 2 * bufb + flagb + zoneb);
   L->err_dev = reinterpret_cast<int*>(L->pool + 2 * bufb + flagb + zoneb + globb);
   L->count_dev = reinterpret_cast<unsigned*>(L->pool + 2 * bufb + flagb + zoneb + globb + 64);
-  e = cudaStreamCreateWithFlags(&L->stream, cudaStreamNonBlocking);
+  L->scalars = globb + sizeof(int) <= ReadBackPool::WORDS ? L->read_back.words() : nullptr;
+  e = L->scalars ? cudaSuccess : cudaErrorMemoryAllocation;
+  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&L->stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) {
     cudaFree(L->pool);
     delete L;
@@ -927,8 +937,7 @@ int tclb_get_quantity(tclb_h L, int q, const int region[6], void* out, double sc
   }
   L->impl->quantity(L, q, vec, r, scale, L->qbuf, s);
   TCLB_CK(cudaGetLastError());
-  TCLB_CK(cudaMemcpyAsync(out, L->qbuf, bytes, cudaMemcpyDeviceToHost, s));
-  TCLB_CK(cudaStreamSynchronize(s));
+  TCLB_CK(L->read_back.copy(out, L->qbuf, bytes, s, L->device));
   return TCLB_OK;
 }
 
@@ -959,8 +968,9 @@ int tclb_energy_enstrophy(tclb_h L, double* out, void* stream) {
   else
     k_energy_enstrophy<float><<<blocks, 256, 0, s>>>(static_cast<const float*>(L->qbuf), L->nx, L->ny, L->nz, acc);
   TCLB_CK(cudaGetLastError());
-  TCLB_CK(cudaMemcpyAsync(out, acc, 2 * sizeof(double), cudaMemcpyDeviceToHost, s));
+  TCLB_CK(cudaMemcpyAsync(L->scalars, acc, 2 * sizeof(double), cudaMemcpyDeviceToHost, s));
   TCLB_CK(cudaStreamSynchronize(s));
+  std::memcpy(out, L->scalars, 2 * sizeof(double));
   return TCLB_OK;
 }
 
@@ -1018,7 +1028,8 @@ int tclb_save(tclb_h L, void* host, size_t bytes, void* stream) {
   cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : L->stream;
   const size_t plane = L->N * L->elem;
   if (L->stride == L->N) {
-    TCLB_CK(cudaMemcpyAsync(host, L->buf[L->cur], bytes, cudaMemcpyDeviceToHost, s));
+    TCLB_CK(L->read_back.copy(host, L->buf[L->cur], bytes, s, L->device));
+    return TCLB_OK;
   } else {
     for (int q = 0; q < L->T->Q; q++)
       TCLB_CK(cudaMemcpyAsync(static_cast<char*>(host) + q * plane,
