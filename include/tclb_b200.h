@@ -195,9 +195,9 @@ int tclb_sync(tclb_h h);
 #define TCLB_LAUNCH_PAIRS 2
 #define TCLB_LAUNCH_TMA 4
 /* With TCLB_LAUNCH_TMA: stage tiles wherever the tile-staged kernel applies,
-   also where d3q19 otherwise takes the register pair kernel (nx % 64 == 0 and
-   rows wider than 256, tiles of fewer than 448 nodes, or fewer than four tiles
-   per resident block: measured faster there). */
+   also where the register pair kernel measured faster: d3q19 with nx % 64 == 0
+   and rows wider than 256, tiles of fewer than 448 nodes, or fewer than four
+   tiles per resident block; d2q9. */
 #define TCLB_LAUNCH_TMA_ALWAYS 8
 int tclb_set_launch(tclb_h h, int bx, int by, int flags);
 /* The launch shape and the paths plain iterations take on this lattice: the

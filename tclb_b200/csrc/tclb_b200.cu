@@ -164,9 +164,8 @@ struct tclb_lattice {
   // 16-bit storage: tile-staged TMA kernel (tma_rows rows per tile; tma[b]
   // describes snapshot b as the source), and its error word in the pool
   int use_tma = 1, tma_ok = 0, tma_rows = 0, tma_grid = 0;
-  // shapes where a model's register pair kernel measured faster (d3q19: rows
-  // wider than 256, under-filled or too few tiles): plain iterations take
-  // that kernel unless tma_always
+  // shapes where a model's register pair kernel measured faster (prepare):
+  // plain iterations take that kernel unless tma_always
   int tma_pref_pairs = 0, tma_always = 0;
   // node pairs of which one node collides and the other not make up at least
   // 1% of the lattice (porous media): the tile-staged kernel of a model with
@@ -226,7 +225,7 @@ Args<R, M::NSET> make_args(const tclb_lattice* L, const void* src, void* dst) {
 // Plain iterations of 16-bit storage take the tile-staged kernel.
 inline bool tma_path(const tclb_lattice* L) {
   return L->use_tma && L->tma_ok && L->tma_grid > 0 &&
-         (L->tma_always || !L->tma_pref_pairs || !(L->use_pairs && L->nx % 64 == 0));
+         (L->tma_always || !L->tma_pref_pairs || !L->use_pairs);
 }
 
 // A kernel launch on stream s whose grid may be scheduled while the previous
@@ -394,15 +393,17 @@ struct Launch {
       }
       const int tiles = L->nz * (L->ny / rows);
       L->tma_grid = std::min(tiles, per_sm * sms);
-      // d3q19 (register pair kernel with identity-rate lanes) takes that kernel
-      // where nx % 64 == 0 and the staged tiles would be under-filled or too
-      // few, as measured on B200 (porous boxes, FP16-shift): rows wider than
-      // 256 (one-row tiles, six consumer warps per block; 384x192x192: 57.7k
-      // against 51.6k MLUPS), tiles of fewer than 448 nodes (192^3: 56.4k
-      // against 50.2k), fewer than four tiles per resident block (64^3: 45.8k
-      // against 27.8k)
+      // Where the register pair kernel measured faster than the staged one (B200,
+      // FP16-shift, us an iteration pairs / staged). d3q19, nx % 64 == 0: rows wider
+      // than 256 (one-row tiles, six consumer warps per block; porous 384 x 192 x
+      // 192 213 / 274), tiles of fewer than 448 nodes (192^3 109 / 141), fewer than
+      // four tiles per resident block (64^3 4.8 / 9.4; 128^3, at fourteen, 35.3 /
+      // 36.1; 256^3 256 / 246). d2q9: every width (512 x 512 3.6 / 4.2, 256 x 1024 4.1 /
+      // 4.9, 512 x 2048 9.7 / 10.4; larger lattices take two iterations per launch).
       if constexpr (M::identity_lanes)
         L->tma_pref_pairs = L->nx % 64 == 0 && (tma_wide(L->nx) || rows * L->nx < 448 || tiles < 4 * per_sm * sms);
+      else if constexpr (M::DIM == 2)
+        L->tma_pref_pairs = 1;
     }
   }
   // Count the node pairs (x, x+1), x even, of which exactly one node
