@@ -1,9 +1,6 @@
 // Device memory -> the caller's host buffer.
 //
-// Small results (Globals, error words, sums) arrive in pinned words of the
-// object that reads them: one asynchronous copy and one wait.
-//
-// Large ones: a copy into pageable memory goes through the driver's staging
+// A copy into pageable memory goes through the driver's staging
 // buffers on one host thread, which also takes the page faults of a fresh
 // array: 3 to 5 GB/s where the link carries 52. Such a copy is cut into parts,
 // one host thread each, with two pinned buffers per thread: while one chunk
@@ -11,16 +8,15 @@
 // admission to read-back of 205 MB: 187 -> 152 ms.) Pinned destinations and
 // copies below 4 MiB go directly.
 //
-// Pinned memory takes about a millisecond to allocate, so the objects of a
-// process share it: 64 KiB of words and, from the first large copy on, 8 MiB
-// of buffers. Both are given back with the last object. The buffers serve one
-// copy at a time, on the device they were made on; a copy that finds them
-// taken goes directly.
+// The objects of a process share the 8 MiB of pinned buffers and the streams.
+// They take some milliseconds to make, so a copy of 16 MiB or more makes them
+// first; they are given back with the last object. They serve one copy at a
+// time, on the device they were made on; a copy that finds them taken goes
+// directly.
 #pragma once
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <bitset>
 #include <cstring>
 #include <mutex>
 #include <thread>
@@ -30,7 +26,6 @@ namespace tclb {
 
 class ReadBackPool {
  public:
-  static constexpr size_t WORDS = 512;  // bytes of an object's pinned words
   static ReadBackPool& get() {
     static ReadBackPool* p = new ReadBackPool;  // never destroyed: the CUDA runtime may be gone by then
     return *p;
@@ -42,39 +37,14 @@ class ReadBackPool {
   void leave() {
     std::lock_guard<std::mutex> l(m_);
     if (--users_ > 0) return;
-    if (slab_) cudaFreeHost(slab_);
-    slab_ = nullptr;
     std::lock_guard<std::mutex> b(busy_);
     release();
   }
-  // Pinned words for an object (nullptr: no memory), and their return.
-  char* take_words() {
-    std::lock_guard<std::mutex> l(m_);
-    if (!slab_ && cudaMallocHost(reinterpret_cast<void**>(&slab_), SLOTS * WORDS) != cudaSuccess) {
-      cudaGetLastError();
-      slab_ = nullptr;
-    }
-    for (size_t i = 0; slab_ && i < SLOTS; i++)
-      if (!used_[i]) {
-        used_[i] = true;
-        return slab_ + i * WORDS;
-      }
-    char* p = nullptr;  // more objects than slots: words of their own
-    if (cudaMallocHost(reinterpret_cast<void**>(&p), WORDS) == cudaSuccess) return p;
-    cudaGetLastError();
-    return nullptr;
-  }
-  void return_words(char* p) {
-    if (!p) return;
-    std::lock_guard<std::mutex> l(m_);
-    if (slab_ && p >= slab_ && p < slab_ + SLOTS * WORDS) used_[(p - slab_) / WORDS] = false;
-    else cudaFreeHost(p);
-  }
-
   // Copy `bytes` after the work enqueued on s; returns when dst holds them.
   cudaError_t copy(void* dst, const void* src, size_t bytes, cudaStream_t s, int device) {
     std::unique_lock<std::mutex> l(busy_, std::defer_lock);
-    if (bytes < PARALLEL_BYTES || pinned(dst) || !l.try_lock() || !prepare(device)) {
+    if (bytes < PARALLEL_BYTES || pinned(dst) || !l.try_lock() || (lanes_.empty() && bytes < FIRST_BYTES) ||
+        !prepare(device)) {
       const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s);
       return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
     }
@@ -103,16 +73,14 @@ class ReadBackPool {
   }
 
  private:
-  static constexpr size_t SLOTS = 128, PARALLEL_BYTES = (size_t)4 << 20, CHUNK = (size_t)512 << 10;
+  static constexpr size_t PARALLEL_BYTES = (size_t)4 << 20, FIRST_BYTES = (size_t)16 << 20, CHUNK = (size_t)512 << 10;
   struct Lane {
     char* buf[2] = {nullptr, nullptr};  // in buffers_
     cudaEvent_t event[2] = {nullptr, nullptr};
     cudaStream_t stream = nullptr;
   };
-  std::mutex m_, busy_;  // the words and the count of objects; the lanes
+  std::mutex m_, busy_;  // the count of objects; the lanes
   int users_ = 0, device_ = -1;
-  char* slab_ = nullptr;
-  std::bitset<SLOTS> used_;
   std::vector<Lane> lanes_;
   char* buffers_ = nullptr;
 
@@ -185,19 +153,12 @@ class ReadBackPool {
 class ReadBack {
  public:
   ReadBack() { ReadBackPool::get().enter(); }
-  ~ReadBack() {
-    ReadBackPool::get().return_words(words_);
-    ReadBackPool::get().leave();
-  }
+  ~ReadBack() { ReadBackPool::get().leave(); }
   ReadBack(const ReadBack&) = delete;
   ReadBack& operator=(const ReadBack&) = delete;
-  char* words() { return words_ ? words_ : words_ = ReadBackPool::get().take_words(); }
   cudaError_t copy(void* dst, const void* src, size_t bytes, cudaStream_t s, int device) {
     return ReadBackPool::get().copy(dst, src, bytes, s, device);
   }
-
- private:
-  char* words_ = nullptr;
 };
 
 }  // namespace tclb

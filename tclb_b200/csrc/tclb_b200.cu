@@ -175,7 +175,10 @@ struct tclb_lattice {
   // 64.5-65.1k; without such pairs, Taylor-Green, parking is 1.3% faster)
   int lanes = 0;
   unsigned* count_dev = nullptr;  // device word for the count
-  char* scalars = nullptr;  // pinned words that small results arrive in
+  // where the Globals and the error word arrive (in pageable memory: a copy of a
+  // few hundred bytes waits for the stream itself, and pinned memory would cost
+  // each lattice milliseconds at its creation)
+  char scalars[1024];
   ReadBack read_back;
   TmaMaps tma[2];
   // plain iterations advanced per launch where there are that many left (1:
@@ -707,8 +710,7 @@ int tclb_create(tclb_h* out, int model, int nx, int ny, int nz, int precision, i
   L->glob_dev = reinterpret_cast<double*>(L->pool + 2 * bufb + flagb + zoneb);
   L->err_dev = reinterpret_cast<int*>(L->pool + 2 * bufb + flagb + zoneb + globb);
   L->count_dev = reinterpret_cast<unsigned*>(L->pool + 2 * bufb + flagb + zoneb + globb + 64);
-  L->scalars = globb + sizeof(int) <= ReadBackPool::WORDS ? L->read_back.words() : nullptr;
-  e = L->scalars ? cudaSuccess : cudaErrorMemoryAllocation;
+  e = globb + sizeof(int) <= sizeof(L->scalars) ? cudaSuccess : cudaErrorInvalidValue;
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&L->stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) {
     cudaFree(L->pool);
