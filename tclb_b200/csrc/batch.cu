@@ -887,13 +887,15 @@ int tclb_batch_set_paths(tclb_batch_h B, int flags) {
   if (flags & ~(TCLB_LAUNCH_PAIRS | TCLB_LAUNCH_TMA | TCLB_BATCH_ADAPTIVE | TCLB_BATCH_GLOBALS_AT_END))
     return bfail(TCLB_ERR_ARG, "unknown path flags");
   if (flags != B->paths) B->tiles_dirty = true;
-  if ((flags ^ B->paths) & TCLB_BATCH_GLOBALS_AT_END) {  // the case descriptors carry the Globals mode
-    BCK(cudaStreamSynchronize(B->stream));
+  if ((flags ^ B->paths) & TCLB_BATCH_GLOBALS_AT_END) {
+    // The case descriptors carry the Globals mode. Only that field is written:
+    // the iterations and launches done and left are the device's, the host copy
+    // holds those of the admission.
     for (size_t s = 0; s < B->cases.size(); s++) {
       if (!B->used_slot[s]) continue;
       B->cases[s].glob_end = (flags & TCLB_BATCH_GLOBALS_AT_END) ? 1 : 0;
-      int rc = upload_case(B, (int)s);
-      if (rc) return rc;
+      BCK(cudaMemcpyAsync(&B->d_cases[s].glob_end, &B->cases[s].glob_end, sizeof(B->cases[s].glob_end),
+                          cudaMemcpyHostToDevice, B->stream));
     }
     BCK(cudaStreamSynchronize(B->stream));
   }

@@ -446,3 +446,30 @@ def test_degenerate_cases_in_a_batch(model, precision):
             assert np.abs(u_b).max() <= 1e-12, s.shape
         assert np.allclose(g_b, g_s, rtol=1e-9 if precision == "fp64" else 1e-4, atol=1e-12), (s.shape, g_b, g_s)
     b.close()
+
+
+# launches done before the change odd and even; cases that advance one and two
+# iterations per launch (the larger is above the size from which two are taken)
+@pytest.mark.parametrize("shape", [(45, 66), (800, 2000)])
+@pytest.mark.parametrize("K,at_end", [(1, False), (4, True), (5, False), (6, True)])
+def test_globals_mode_changed_between_steps(shape, K, at_end):
+    """A case that has iterations left keeps its count and its state; a finished one stays finished."""
+    ny, nx = shape
+    flags = cases.channel_disc_d2q9(nx, ny, 6, nx // 4, ny // 2)
+    specs = [CaseSpec(flags, {"Viscosity": 0.02}, {0: {"VelocityX": 0.01}}, n) for n in (2 * K + 3, K)]
+    b = Batch("d2q9", "fp32", budget_bytes=2 << 30)
+    b.set_paths(globals_at_end=at_end)
+    b.set_launch(64, 16, K)
+    ids = [b.add_case(s) for s in specs]
+    b.step()
+    b.sync()
+    done = b.quantity(ids[1], "U")
+    b.set_paths(globals_at_end=not at_end)
+    b.run_to_completion()
+    for cid, s in zip(ids, specs):
+        assert b.poll(cid) == (s.niter, 0)
+        u, g = run_single("d2q9", s, "fp32")
+        assert rel_l2(b.quantity(cid, "U"), u) <= TOL_U["fp32"]
+        assert np.allclose(b.globals(cid), g, rtol=1e-6, atol=1e-9)  # FP64 sums in another order
+    assert np.array_equal(b.quantity(ids[1], "U"), done)
+    b.close()
