@@ -19,6 +19,7 @@
 #include <utility>
 
 #include "../../include/tclb_b200.h"
+#include "launch_rules.h"
 #include "lbm_rows.cuh"
 #include "lbm_tma.cuh"
 #include "read_back.h"
@@ -488,22 +489,6 @@ const Impl* impl_for(int model, int precision, int storage) {
 
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
-// Block of the one-node kernel: in 3D the widest multiple of 32 that divides
-// the row (a block of whole rows touches the fewest HBM pages, and none of its
-// threads is idle), two or more rows while it has fewer than 128 threads; in
-// 2D, where the lattices of this kernel live in L2, 32 x 4. Measured (us an
-// iteration, 128 x 2 before and the shape chosen now): d3q19 192 x 96 x 96 FP32
-// 49.7/44.6, 160^3 FP32 108.4/100.8, 256^3 FP32 399/392; d3q27 256^3 FP32
-// 580/566, 192 x 64 x 64 FP32 31.4/29.0; d2q9 1024 x 256 FP64 4.82/4.67.
-void block_shape(tclb_lattice* L) {
-  L->bx = 32;
-  if (L->nz > 1)
-    for (int b = 64; b <= 256; b += 32)
-      if (L->nx % b == 0) L->bx = b;
-  L->by = L->bx >= 128 ? 1 : std::max(1, 128 / L->bx);
-  if ((L->ny + L->by - 1) / L->by > 65535) L->by = 256 / L->bx;  // grid limit
-}
-
 // Tensor maps of the tile-staged kernel (16-bit storage, nx a multiple of 32
 // and at most 512, R <= 512 / nx rows per tile dividing ny). When anything
 // does not fit, tma_ok stays 0 and the register kernels run.
@@ -717,7 +702,9 @@ int tclb_create(tclb_h* out, int model, int nx, int ny, int nz, int precision, i
     delete L;
     return fail(TCLB_ERR_CUDA, std::string("stream create failed: ") + cudaGetErrorString(e));
   }
-  block_shape(L);
+  const BlockShape shape = block_shape(nx, ny, nz);
+  L->bx = shape.bx;
+  L->by = shape.by;
   // settings defaults (src/Solver.cpp.Rt:276-281) and zonal defaults (:393)
   L->settings.assign(T->nsettings, 0.0);
   for (int i = 0; i < T->nsettings; i++)

@@ -1,0 +1,67 @@
+"""The rules that choose a launch, compiled for the host from the header the library includes."""
+import ctypes
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from tclb_b200 import models as M
+from tclb_b200.lattice import Lattice
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "tclb_b200", "csrc")
+SOURCE = """
+#include "launch_rules.h"
+extern "C" void shape(int nx, int ny, int nz, int* out) {
+  const tclb::BlockShape s = tclb::block_shape(nx, ny, nz);
+  out[0] = s.bx;
+  out[1] = s.by;
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def rules(tmp_path_factory):
+    d = tmp_path_factory.mktemp("rules")
+    (d / "rules.cpp").write_text(SOURCE)
+    subprocess.check_call(["g++", "-std=c++17", "-O1", "-Wall", "-Werror", "-shared", "-fPIC", "-I", CSRC,
+                           "-o", str(d / "rules.so"), str(d / "rules.cpp")])
+    return ctypes.CDLL(str(d / "rules.so"))
+
+
+# rows a launch has always taken: blocks of 128 x 2, 64 x 4 and 32 x 8 threads by the width
+@pytest.mark.parametrize("nz", [1, 2])
+@pytest.mark.parametrize("nx,rows", [(17, 524280), (32, 524280), (64, 262140), (96, 262140), (128, 131070),
+                                     (160, 131070), (192, 131070), (224, 131070), (256, 131070), (300, 131070)])
+def test_every_height_fits_the_grid(rules, nx, rows, nz):
+    out = (ctypes.c_int * 2)()
+    for ny in (1, 2, 65535, 65536, 70000, 131070, 131071, 262140, 262141, rows):
+        if ny > rows:
+            continue
+        rules.shape(nx, ny, nz, out)
+        bx, by = out
+        assert bx % 32 == 0 and by >= 1 and bx * by <= 256
+        assert (ny + by - 1) // by <= 65535, (nx, ny, bx, by)
+
+
+@pytest.mark.gpu
+def test_more_rows_than_a_grid_of_one_row_blocks():
+    """160 wide, whole-row blocks while they fit: the height does not, and the result is that of blocks of 64 x 4."""
+    nx, ny, nz = 160, 65540, 2
+    m = M.get("d3q19")
+    flags = np.full((nz, ny, nx), m.flag("MRT"), np.uint16)
+    flags[np.random.default_rng(1).random(flags.shape) < 0.05] = m.flag("Wall")
+    out = []
+    for shape in (None, (64, 4)):
+        g = Lattice("d3q19", nx, ny, nz, precision="fp32")
+        if shape:
+            g.set_launch(*shape)
+        g.set_flags(flags)
+        g.SetSetting("nu", 0.05)
+        g.SetSetting("InletVelocity", 0.02)
+        g.Init()
+        g.Iterate(3, M.ITER_NORM)
+        out.append(g.GetQuantity("U"))
+        g.close()
+    assert np.isfinite(out[0]).all() and np.abs(out[0]).max() > 1e-3
+    assert np.array_equal(out[0], out[1])
