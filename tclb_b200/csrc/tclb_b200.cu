@@ -702,7 +702,7 @@ int tclb_create(tclb_h* out, int model, int nx, int ny, int nz, int precision, i
     delete L;
     return fail(TCLB_ERR_CUDA, std::string("stream create failed: ") + cudaGetErrorString(e));
   }
-  const BlockShape shape = block_shape(nx, ny, nz);
+  const BlockShape shape = block_shape(T->Q, (int)L->elem, nx, ny, nz);
   L->bx = shape.bx;
   L->by = shape.by;
   // settings defaults (src/Solver.cpp.Rt:276-281) and zonal defaults (:393)

@@ -12,8 +12,8 @@ from tclb_b200.lattice import Lattice
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "tclb_b200", "csrc")
 SOURCE = """
 #include "launch_rules.h"
-extern "C" void shape(int nx, int ny, int nz, int* out) {
-  const tclb::BlockShape s = tclb::block_shape(nx, ny, nz);
+extern "C" void shape(int q, int elem, int nx, int ny, int nz, int* out) {
+  const tclb::BlockShape s = tclb::block_shape(q, elem, nx, ny, nz);
   out[0] = s.bx;
   out[1] = s.by;
 }
@@ -35,13 +35,28 @@ def rules(tmp_path_factory):
                                      (160, 131070), (192, 131070), (224, 131070), (256, 131070), (300, 131070)])
 def test_every_height_fits_the_grid(rules, nx, rows, nz):
     out = (ctypes.c_int * 2)()
-    for ny in (1, 2, 65535, 65536, 70000, 131070, 131071, 262140, 262141, rows):
-        if ny > rows:
-            continue
-        rules.shape(nx, ny, nz, out)
-        bx, by = out
-        assert bx % 32 == 0 and by >= 1 and bx * by <= 256
-        assert (ny + by - 1) // by <= 65535, (nx, ny, bx, by)
+    for q, elem in [(9, 4), (9, 8)] if nz == 1 else [(19, 4), (19, 8), (27, 4)]:
+        for ny in (1, 2, 65535, 65536, 70000, 131070, 131071, 262140, 262141, rows):
+            if ny > rows:
+                continue
+            rules.shape(q, elem, nx, ny, nz, out)
+            bx, by = out
+            assert bx % 32 == 0 and by >= 1 and bx * by <= 256
+            assert (ny + by - 1) // by <= 65535, (nx, ny, bx, by)
+
+
+# both sides of the node counts (4 and 8 blocks of 128 for each of 148 SMs) and of the width that have a shape of
+# their own
+@pytest.mark.parametrize("q,elem,size,shape", [
+    (9, 4, (256, 295, 1), (32, 4)), (9, 4, (256, 296, 1), (32, 8)), (9, 4, (512, 256, 1), (32, 8)),
+    (9, 4, (256, 591, 1), (32, 8)), (9, 4, (256, 592, 1), (32, 4)), (9, 8, (512, 256, 1), (32, 4)),
+    (19, 4, (224, 64, 64), (32, 4)), (19, 4, (448, 64, 64), (64, 2)), (19, 8, (224, 64, 64), (224, 1)),
+    (27, 4, (224, 64, 64), (224, 1)), (19, 4, (192, 64, 64), (192, 1)), (19, 4, (256, 64, 64), (256, 1)),
+    (27, 4, (128, 64, 64), (128, 1)), (19, 4, (64, 64, 64), (64, 2)), (19, 4, (33, 64, 64), (32, 4))])
+def test_block_of_the_one_node_kernel(rules, q, elem, size, shape):
+    out = (ctypes.c_int * 2)()
+    rules.shape(q, elem, *size, out)
+    assert tuple(out) == shape
 
 
 @pytest.mark.gpu
