@@ -187,8 +187,9 @@ int tclb_sync(tclb_h h);
    stage tiles of whole rows in shared memory with TMA on plain iterations
    (on by default; it takes precedence over PAIRS) when nx is a multiple of 32
    up to 512 (tiles of whole rows, at most 512 nodes, the number of rows
-   dividing ny). bx, by shape the one-node kernel of widths that are a
-   multiple of 32.
+   dividing ny). bx, by shape the one-node kernel of plain iterations at
+   widths that are a multiple of 32, and the kernels that initialise a lattice;
+   iterations with Globals and other widths have blocks of their own.
    A staging wait that runs out (about a second) is reported as TCLB_ERR_CUDA
    by the next tclb_sync or Globals-reading tclb_iterate. */
 #define TCLB_LAUNCH_GRAPHS 1
@@ -197,7 +198,8 @@ int tclb_sync(tclb_h h);
 /* With TCLB_LAUNCH_TMA: stage tiles wherever the tile-staged kernel applies,
    also where the register pair kernel measured faster: d3q19 with nx % 64 == 0
    and rows wider than 256, tiles of fewer than 448 nodes, or fewer than four
-   tiles per resident block; d2q9. */
+   tiles per resident block; d2q9 below 2.1 million nodes, 2.6 with tiles of
+   fewer than 320, and with tiles of fewer than 192. */
 #define TCLB_LAUNCH_TMA_ALWAYS 8
 int tclb_set_launch(tclb_h h, int bx, int by, int flags);
 /* The launch shape and the paths plain iterations take on this lattice: the

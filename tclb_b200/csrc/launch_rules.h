@@ -1,6 +1,7 @@
 // Rules of the launches that need no device: plain C++.
 #pragma once
 #include <algorithm>
+#include <cstddef>
 
 namespace tclb {
 
@@ -39,6 +40,19 @@ inline BlockShape block_shape(int q, int elem, int nx, int ny, int nz) {
   }
   if ((ny - 1) / by + 1 > GRID_ROWS) return {32, 8};
   return {bx, by};
+}
+
+// Single launches of d2q9 in 16 bits: whether in pairs of nodes rather than staged
+// in tiles of `tile` nodes. Pairs are faster while two snapshots and the node
+// types take less than two thirds of the L2, and always where the tiles are too
+// small. Us an iteration, pairs / staged: 256 x 1024 in tiles of 512 3.3/4.3, 256 x
+// 4096 8.7/9.2, 256 x 7800 15.1/15.0, 256 x 9400 19.7/17.8, 256 x 23400 55.7/40.5; in
+// tiles of 256 256 x 8600 19.7/20.5, 256 x 10200 24.7/24.3, 256 x 23400 55.6/49.2;
+// 192 x 31200 of 192 55.8/49.2, 160 x 37500 of 160 61.5/57.4, 96 x 62500 of 96 61.5/82.7,
+// 32 x 187500 of 32 61.5/184.4; with 10% of the nodes solid 256 x 23400 of 512
+// 64.2/53.4, of 256 63.8/61.5, 192 of 192 64.0/65.5, 160 of 160 71.3/77.9.
+inline bool pairs_pay_2d(std::size_t nodes, int tile) {
+  return tile < 192 || nodes < (tile >= 320 ? 2100000u : 2600000u);
 }
 
 }  // namespace tclb

@@ -402,12 +402,11 @@ struct Launch {
       // than 256 (one-row tiles, six consumer warps per block; porous 384 x 192 x
       // 192 213 / 274), tiles of fewer than 448 nodes (192^3 109 / 141), fewer than
       // four tiles per resident block (64^3 4.8 / 9.4; 128^3, at fourteen, 35.3 /
-      // 36.1; 256^3 256 / 246). d2q9: every width (512 x 512 3.6 / 4.2, 256 x 1024 4.1 /
-      // 4.9, 512 x 2048 9.7 / 10.4; larger lattices take two iterations per launch).
+      // 36.1; 256^3 256 / 246).
       if constexpr (M::identity_lanes)
         L->tma_pref_pairs = L->nx % 64 == 0 && (tma_wide(L->nx) || rows * L->nx < 448 || tiles < 4 * per_sm * sms);
       else if constexpr (M::DIM == 2)
-        L->tma_pref_pairs = 1;
+        L->tma_pref_pairs = pairs_pay_2d(L->N, rows * L->nx);
     }
   }
   // Count the node pairs (x, x+1), x even, of which exactly one node

@@ -17,6 +17,7 @@ extern "C" void shape(int q, int elem, int nx, int ny, int nz, int* out) {
   out[0] = s.bx;
   out[1] = s.by;
 }
+extern "C" int pairs_pay_2d(long long nodes, int tile) { return tclb::pairs_pay_2d(nodes, tile); }
 """
 
 
@@ -57,6 +58,14 @@ def test_block_of_the_one_node_kernel(rules, q, elem, size, shape):
     out = (ctypes.c_int * 2)()
     rules.shape(q, elem, *size, out)
     assert tuple(out) == shape
+
+
+@pytest.mark.parametrize("tile,nodes,pairs", [
+    (512, 2_099_999, 1), (512, 2_100_000, 0), (320, 2_100_000, 0), (256, 2_100_000, 1), (256, 2_599_999, 1),
+    (256, 2_600_000, 0), (192, 2_600_000, 0), (160, 9_000_000, 1), (32, 9_000_000, 1)])
+def test_pairs_or_staged_single_launches(rules, tile, nodes, pairs):
+    rules.pairs_pay_2d.argtypes = [ctypes.c_longlong, ctypes.c_int]
+    assert rules.pairs_pay_2d(nodes, tile) == pairs
 
 
 @pytest.mark.gpu

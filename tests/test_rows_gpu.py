@@ -2,6 +2,7 @@
 one iteration per launch, whose kernels the other tests hold to the oracle."""
 import numpy as np
 import pytest
+import torch
 
 from tclb_b200 import models as M
 from tclb_b200.batch import Batch, CaseSpec
@@ -15,6 +16,27 @@ TYPES = ["Wall", "Solid", "WVelocity", "EPressure", "NSymmetry", "EVelocity", "W
 PARAMS = [("setting", "Viscosity", 0.05), ("setting", "S3", 0.3), ("setting", "S4", 0.2),
           ("setting", "GravitationX", 1e-6), ("setting", "GravitationY", -2e-6),
           ("zone", "VelocityX", 0.02, 1), ("zone", "Pressure", 0.01, 1)]
+BOUNDARY, SOLID = M.get("d2q9").groups["BOUNDARY"][0], M.get("d2q9").flag("Solid")
+
+
+def kernels(run):
+    """Names of the kernels that run() launches (graph replays included)."""
+    torch.zeros(1, device="cuda")
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as p:
+        run()
+    return " ".join(e.key for e in p.key_averages())
+
+
+def start(nx, ny, precision, storage, flags, seed):
+    """A lattice from a perturbed flow, with forces and boundary values of its own."""
+    rng = np.random.default_rng(seed)
+    real = np.float64 if precision == "fp64" else np.float32
+    g = Lattice("d2q9", nx, ny, precision=precision, storage=storage)
+    g.set_flags(flags)
+    apply_params(g, PARAMS)
+    g.init_equilibrium((1 + 0.01 * rng.standard_normal(nx * ny)).astype(real),
+                       (0.02 * rng.standard_normal((nx * ny, 3))).astype(real))
+    return g
 
 
 # widths that do and do not divide into strips (60 columns in pairs, 30 one per
@@ -63,6 +85,23 @@ def test_graph_replays_of_two_iterations():
         out.append(g.GetQuantity("U"))
         g.close()
     assert np.allclose(out[0], out[1], rtol=0, atol=1e-6)
+
+
+# 16-bit rows that can be staged: in pairs while the lattice stays in L2, staged beyond, the same bits
+@pytest.mark.parametrize("nx,ny,kernel", [(256, 8202, "k_iterate_pair"), (256, 8204, "k_iterate_tma"),
+                                          (256, 10155, "k_iterate_pair"), (256, 10157, "k_iterate_tma"),
+                                          (96, 40001, "k_iterate_pair")])
+def test_single_launches_of_staged_widths(nx, ny, kernel):
+    fl = random_flags("d2q9", (1, ny, nx), TYPES[:4], zones=2, seed=4, p_type=0.05)
+    out = []
+    for launch in ({}, {"tma_always": True}, {"use_tma": False}):
+        g = start(nx, ny, "fp32", "fp16s", fl, 6)
+        if launch:
+            g.set_launch(32, 4, **launch)
+        assert (kernel in kernels(lambda: ([g.Iterate(1, M.ITER_NORM) for _ in range(3)], g.sync()))) or launch
+        out.append(g.save().tobytes())
+        g.close()
+    assert out[0] == out[1] == out[2]
 
 
 # iterations per replay even, odd and one; iteration counts that end anywhere in
