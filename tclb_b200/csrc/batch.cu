@@ -486,7 +486,7 @@ int rebuild_tiles(tclb_batch* B) {
       const bool two = rows_case_of(B, s);
       if (!live(B, s) || (staged(B, C) || two) != (pass == 1)) continue;
       if (two) {
-        const int cols = B->elem == 8 ? rows_columns<false>(2) : rows_columns<true>(2);
+        const int cols = rows_columns(B->elem < 8, 2);
         for (int y = 0; y < C.ny; y += ROWS_HEIGHT)
           for (int x = 0; x * cols < C.nx; x++) rows.push_back({(int)s, x, y});
         for (int y = 0; y < C.ny; y += h)

@@ -42,6 +42,58 @@ inline BlockShape block_shape(int q, int elem, int nx, int ny, int nz) {
   return {bx, by};
 }
 
+// k_iterate_rows: the columns of a strip (PAIR: two nodes per lane), and those
+// lost at either edge. One node per lane pulls
+// its first row from the neighbouring columns directly; two nodes per lane
+// load aligned pairs and shift them by shuffles in the first stage too, and
+// store aligned pairs (an even count lost).
+constexpr int rows_lost(bool pair, int T) { return pair ? (T + 1) / 2 * 2 : T - 1; }
+constexpr int rows_lanes(bool pair) { return pair ? 64 : 32; }
+constexpr int rows_columns(bool pair, int T) { return rows_lanes(pair) - 2 * rows_lost(pair, T); }
+
+// Nodes from which two iterations per launch are faster than two launches of
+// the one-iteration kernels, which have one warp per 32 or 64 nodes to hide
+// latency with and live in L2 at these sizes. Measured at 1024 x 256, 2048 x
+// 512 and 4096 x 1024 (us an iteration, one launch each against this kernel):
+// FP64 4.8/5.6, 22.5/17.4, 92.7/57.9; FP32 3.9/5.2, 10.2/10.4, 50.0/33.3;
+// 16 bits 3.7/5.2, 8.1/10.8, 35.9/29.1.
+inline std::size_t rows_min_nodes(std::size_t elem) { return elem == 8 ? 700000 : (elem == 4 ? 1500000 : 2500000); }
+
+// Whether a lattice of `nodes` nodes, nx wide, takes them. Above rows_min_nodes
+// it is the share of the strips' columns that are nodes of the lattice (94% of a
+// width that strips divide, 50% of 64 in pairs) that decides, and whether 1% of
+// the node pairs or more are `mixed`, one node colliding and the other not: with
+// two nodes per lane that of the other is parked across the collision, twice a
+// launch, and the one-node kernels hardly slow down. Single launches
+// against this kernel, us an iteration, clean and with 10% of the nodes solid:
+// FP32 pairs 1024 x 1560 19.1/11.9 and 19.9/17.3, 1024 x 1660 20.4/14.0 and
+// 21.2/22.9, 1024 x 2150 28.2/17.6 and 28.8/27.2; 192 x 11460 28.2/18.6 and
+// 28.9/28.8; 128 x 32800 49.7/35.2 and 51.0/54.4; 64 x 25000 18.5/18.3 and
+// 19.6/28.4, 62 x 25800 18.9/18.6, 30 x 53300 18.8/20.0.
+// FP32, one node per lane, 255 x 6270 19.0/15.3 and 19.7/17.6, 99 x 16200 19.0/16.9
+// and 19.8/20.1, 91 x 17600 18.9/17.8 and 19.9/21.2, 61 x 26200 19.0/19.8.
+// FP64 96 x 7400 13.4/11.7 and 13.9/13.9, 64 x 11700 14.4/13.3 and 14.9/15.7, 64 x
+// 18750 27.9/20.3 and 28.2/23.7, 32 x 23400 13.8/15.8, 32 x 62500 45.2/40.2 and
+// 45.3/47.8.
+// 16 bits, single launches in pairs: 1024 x 2460 24.2/17.8 and 28.6/26.7, 190 x
+// 13700 26.1/20.9, 40 x 65000 26.0/24.1 and 30.8/35.5, 66 x 39400 25.9/28.7. Staged
+// in tiles of `tile` nodes (0: not staged) they are faster, the more so the
+// fuller the tile (of 512): 512 x 11700 40.4/38.5 and 53.5/57.8, 256 x 23400 in
+// tiles of 512 40.5/41.7 and 53.4/62.7, of 256 49.2/41.7 and 61.5/62.8; 192 x
+// 31200 of 384 41.5/44.6, of 192 49.2/44.6; 352 x 17000 47.2/37.2 and 63.5/55.8; 128
+// x 46900 of 256 49.2/49.3 and 61.5/74.1.
+inline bool rows_pay(std::size_t elem, int nx, std::size_t nodes, bool mixed, int tile) {
+  const bool pair = elem < 8 && nx % 2 == 0;
+  if (nodes < rows_min_nodes(elem) || (elem == 2 && !pair)) return false;
+  const long long strips = (nx - 1) / rows_columns(pair, 2) + 1;
+  const int share = (int)(100LL * nx / (strips * rows_lanes(pair)));  // percent
+  if (elem == 8) return nodes >= 1100000 ? share >= (mixed ? 60 : 48) : share >= (mixed ? 75 : 60);
+  if (elem == 4 && pair) return mixed ? share >= 75 && nodes >= 2200000 : share >= 48;
+  if (elem == 4) return share >= (mixed ? 77 : 65);
+  if (tile == 0) return share >= (mixed ? 80 : 60);
+  return share >= (tile >= 384 || mixed ? 83 : 70) && !(mixed && tile >= 512);
+}
+
 // Single launches of d2q9 in 16 bits: whether in pairs of nodes rather than staged
 // in tiles of `tile` nodes. Pairs are faster while two snapshots and the node
 // types take less than two thirds of the L2, and always where the tiles are too

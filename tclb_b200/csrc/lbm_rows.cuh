@@ -17,6 +17,7 @@
 // on the same values, and 16-bit storage rounds between the stages as a
 // store and a load would, so one launch of T gives the bits of T launches.
 #pragma once
+#include "launch_rules.h"
 #include "lbm_kernels.cuh"
 
 namespace tclb {
@@ -29,23 +30,6 @@ constexpr int ROWS_AHEAD = 2;   // rows staged ahead of the one updated
 // 4096 x 1024: 8 rows 33.3 us an iteration, 16 36.3, 32 47.4; 4096 x 4096:
 // 115, 120, 132).
 constexpr int ROWS_HEIGHT = 8;
-// Nodes from which two iterations per launch are faster than two launches of
-// the one-iteration kernels, which have one warp per 32 or 64 nodes to hide
-// latency with and live in L2 at these sizes. Measured at 1024 x 256, 2048 x
-// 512 and 4096 x 1024 (us an iteration, one launch each against this kernel):
-// FP64 4.8/5.6, 22.5/17.4, 92.7/57.9; FP32 3.9/5.2, 10.2/10.4, 50.0/33.3;
-// 16 bits 3.7/5.2, 8.1/10.8, 35.9/29.1.
-inline size_t rows_min_nodes(size_t elem) { return elem == 8 ? 700000 : (elem == 4 ? 1500000 : 2500000); }
-
-// Columns of a strip, and those lost at either edge. One node per lane pulls
-// its first row from the neighbouring columns directly; two nodes per lane
-// load aligned pairs and shift them by shuffles in the first stage too, and
-// store aligned pairs (an even count lost).
-template <bool PAIR>
-__host__ __device__ constexpr int rows_lost(int T) { return PAIR ? (T + 1) / 2 * 2 : T - 1; }
-template <bool PAIR>
-__host__ __device__ constexpr int rows_columns(int T) { return (PAIR ? 64 : 32) - 2 * rows_lost<PAIR>(T); }
-
 // A lane's one or two nodes of a population as stored.
 template <class St>
 struct RowPair {  // 16-bit storage: two values in a word
@@ -117,10 +101,10 @@ __device__ __forceinline__ void rows_walk(const AR& a, const A& P, int strip, in
   static_assert(PAIR || !St::shifted, "one node per lane: 32- and 64-bit storage");
   using Row = std::conditional_t<PAIR, RowPair<St>, RowOne<St>>;
   using Raw = typename Row::Raw;
-  constexpr int Q = M::Q, LOST = rows_lost<PAIR>(T), PER = PAIR ? 2 : 1;
+  constexpr int Q = M::Q, LOST = rows_lost(PAIR, T), PER = PAIR ? 2 : 1;
   const int lane = threadIdx.x & 31;
   const int nx = a.nx, ny = a.ny;
-  const int x0 = strip * rows_columns<PAIR>(T) - LOST + PER * lane;  // not wrapped
+  const int x0 = strip * rows_columns(PAIR, T) - LOST + PER * lane;  // not wrapped
   const bool mine = PER * lane >= LOST && PER * lane < 32 * PER - LOST && x0 < nx;
   int x = x0 % nx;
   if (x < 0) x += nx;

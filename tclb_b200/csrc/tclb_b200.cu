@@ -169,12 +169,13 @@ struct tclb_lattice {
   // plain iterations take that kernel unless tma_always
   int tma_pref_pairs = 0, tma_always = 0;
   // node pairs of which one node collides and the other not make up at least
-  // 1% of the lattice (porous media): the tile-staged kernel of a model with
-  // identity-rate lanes runs the other node at identity rates instead of
-  // parking it (measured on B200, d3q19 porous 256^3 FP16-shift: 2% solids
+  // 1% of the lattice (porous media; counted where a choice depends on it):
+  // fewer 2D lattices take two iterations per launch (rows_pay), and the
+  // tile-staged kernel of a model with identity-rate lanes runs the other node
+  // at identity rates instead of parking it (measured on B200, d3q19 porous 256^3 FP16-shift: 2% solids
   // 66.1k -> 67.5k MLUPS, 8.5% 62.1k -> 64.6-64.9k, 15% 61.3-61.6k ->
   // 64.5-65.1k; without such pairs, Taylor-Green, parking is 1.3% faster)
-  int lanes = 0;
+  int mixed = 0;
   unsigned* count_dev = nullptr;  // device word for the count
   // where the Globals and the error word arrive (in pageable memory: a copy of a
   // few hundred bytes waits for the stream itself, and pinned memory would cost
@@ -182,9 +183,6 @@ struct tclb_lattice {
   char scalars[1024];
   ReadBack read_back;
   TmaMaps tma[2];
-  // plain iterations advanced per launch where there are that many left (1:
-  // one at a time)
-  int steps = 1;
   int glob_grid = 0;  // blocks of a Globals iteration (set by the first)
   int* err_dev = nullptr;
   // failure-path test of the tile-staged kernel (tclb_set_fault_injection):
@@ -195,7 +193,7 @@ struct tclb_lattice {
 
 struct Impl {
   void (*iterate)(tclb_lattice*, bool, cudaStream_t);
-  void (*iterate_steps)(tclb_lattice*, cudaStream_t);  // L->steps plain iterations, from buf[cur] to buf[1 - cur]
+  void (*iterate_two)(tclb_lattice*, cudaStream_t);  // two plain iterations of a 2D lattice, from buf[cur] to buf[1 - cur]
   int (*flags_changed)(tclb_lattice*);  // after new node types: the kernel choices that depend on them
   void (*init)(tclb_lattice*, cudaStream_t);
   void (*quantity)(tclb_lattice*, int, int, const int*, double, void*, cudaStream_t);
@@ -252,7 +250,7 @@ void launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cuda
 
 template <class M>
 inline bool tma_lanes(const tclb_lattice* L) {
-  return M::identity_lanes && L->lanes;
+  return M::identity_lanes && L->mixed;
 }
 
 inline dim3 grid_of(const tclb_lattice* L) {
@@ -355,25 +353,20 @@ struct Launch {
       P.s[i] = static_cast<const E*>(a.src) + (size_t)i * L->stride;
       P.d[i] = static_cast<E*>(a.dst) + (size_t)i * L->stride;
     }
-    constexpr int C = rows_columns<PAIR>(2);
+    constexpr int C = rows_columns(PAIR, 2);
     const int strips = (L->nx + C - 1) / C, warps = strips * ((L->ny + ROWS_HEIGHT - 1) / ROWS_HEIGHT);
     launch_pdl(k_iterate_rows<M, R, St, 2, PAIR>, dim3((warps + ROWS_WARPS - 1) / ROWS_WARPS), dim3(32 * ROWS_WARPS),
                0, s, a, P, strips, warps);
   }
-  static void iterate_steps(tclb_lattice* L, cudaStream_t s) {
+  static void iterate_two(tclb_lattice* L, cudaStream_t s) {
     if constexpr (rows_pair) {
       if (L->nx % 2 == 0) return launch_rows<true>(L, s);
     }
     if constexpr (rows_one) launch_rows<false>(L, s);
   }
-  static void prepare_steps(tclb_lattice* L) {
-    L->steps = 1;
-    if (M::DIM == 2 && L->N >= rows_min_nodes(sizeof(typename St::T)) && (rows_one || L->nx % 2 == 0)) L->steps = 2;
-  }
   // Once at creation: the dynamic shared-memory limit and persistent grid of the
   // tile-staged kernel (resident blocks per SM x SMs, at most one per tile).
   static void prepare(tclb_lattice* L) {
-    prepare_steps(L);
     using T = typename St::T;
     if constexpr (sizeof(T) == 2) {
       if (!L->tma_ok) return;
@@ -409,12 +402,14 @@ struct Launch {
         L->tma_pref_pairs = pairs_pay_2d(L->N, rows * L->nx);
     }
   }
-  // Count the node pairs (x, x+1), x even, of which exactly one node
-  // collides; with 16-bit storage and identity-rate lanes, set L->lanes.
+  // Count the node pairs (2p, 2p + 1) of the flat index (of one row when nx is
+  // even) of which exactly one node collides; set L->mixed.
   static int flags_changed(tclb_lattice* L) {
-    L->lanes = 0;
-    if constexpr (M::identity_lanes && sizeof(typename St::T) == 2) {
-      if (L->nx % 2) return TCLB_OK;
+    using T = typename St::T;
+    constexpr bool staged_lanes = M::identity_lanes && sizeof(T) == 2;
+    L->mixed = 0;
+    if constexpr (staged_lanes || M::DIM == 2) {
+      if (staged_lanes ? L->nx % 2 != 0 : L->N < rows_min_nodes(sizeof(T))) return TCLB_OK;
       const unsigned npairs = (unsigned)(L->N / 2);
       TCLB_CK(cudaMemsetAsync(L->count_dev, 0, sizeof(unsigned), L->stream));
       k_count_mixed_pairs<M><<<std::min<unsigned>((npairs + 255) / 256, 1184), 256, 0, L->stream>>>(
@@ -423,7 +418,7 @@ struct Launch {
       unsigned mixed = 0;
       TCLB_CK(cudaMemcpyAsync(&mixed, L->count_dev, sizeof(unsigned), cudaMemcpyDeviceToHost, L->stream));
       TCLB_CK(cudaStreamSynchronize(L->stream));
-      L->lanes = (unsigned long long)mixed * 100 >= npairs ? 1 : 0;
+      L->mixed = (unsigned long long)mixed * 100 >= npairs ? 1 : 0;
     }
     return TCLB_OK;
   }
@@ -458,7 +453,7 @@ struct Launch {
       for (size_t n = 0; n < N; n++) p[(size_t)q * stride + n] = St::from_double(in[(size_t)q * N + n], M::w(q));
   }
   static const Impl* get() {
-    static const Impl impl = {iterate, iterate_steps, flags_changed, init,    quantity, equilibrium, color,
+    static const Impl impl = {iterate, iterate_two, flags_changed, init,    quantity, equilibrium, color,
                               to_double, from_double, prepare, sizeof(R)};
     return &impl;
   }
@@ -548,13 +543,14 @@ void drop_graphs(tclb_lattice* L) {
 // kernel: the arithmetic, and so the result, does not depend on how a run is
 // cut into calls.
 int plain_steps(tclb_lattice* L, int n, cudaStream_t s) {
-  const bool packed = tma_path(L) || (L->use_pairs && L->nx % 2 == 0);
+  const bool staged = tma_path(L), packed = staged || (L->use_pairs && L->nx % 2 == 0);
   const bool set = L->tma_always || L->fault_tile >= 0 || L->wait_cycles != TMA_WAIT_CYCLES;  // staging asked for
-  const bool many = L->steps > 1 && n >= L->steps && (L->elem > 2 || (packed && !set));
-  if (many) L->impl->iterate_steps(L, s);
+  const bool two = n >= 2 && L->T->dim == 2 && (L->elem > 2 || (packed && !set)) &&
+                   rows_pay(L->elem, L->nx, L->N, L->mixed, staged ? L->tma_rows * L->nx : 0);
+  if (two) L->impl->iterate_two(L, s);
   else L->impl->iterate(L, false, s);
   L->cur = 1 - L->cur;
-  return many ? L->steps : 1;
+  return two ? 2 : 1;
 }
 
 // Capture GRAPH_CHUNK plain iterations starting from the current snapshot.
@@ -762,10 +758,10 @@ int tclb_set_flags(tclb_h L, const uint16_t* flags, int dx, int dy, int dz, int 
     }
   }
   TCLB_CK(cudaStreamSynchronize(L->stream));
-  const int lanes = L->lanes;
+  const int mixed = L->mixed;
   const int rc = L->impl->flags_changed(L);
   if (rc != TCLB_OK) return rc;
-  if (L->lanes != lanes) drop_graphs(L);  // the captured launches name the other kernel
+  if (L->mixed != mixed) drop_graphs(L);  // the captured launches name the other kernel
   return TCLB_OK;
 }
 

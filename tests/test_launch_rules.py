@@ -17,6 +17,9 @@ extern "C" void shape(int q, int elem, int nx, int ny, int nz, int* out) {
   out[0] = s.bx;
   out[1] = s.by;
 }
+extern "C" int rows_pay(int elem, int nx, long long nodes, int mixed, int tile) {
+  return tclb::rows_pay(elem, nx, nodes, mixed != 0, tile);
+}
 extern "C" int pairs_pay_2d(long long nodes, int tile) { return tclb::pairs_pay_2d(nodes, tile); }
 """
 
@@ -58,6 +61,32 @@ def test_block_of_the_one_node_kernel(rules, q, elem, size, shape):
     out = (ctypes.c_int * 2)()
     rules.shape(q, elem, *size, out)
     assert tuple(out) == shape
+
+
+# (bytes per value, width, nodes): taken when clean, when mixed; and the same where single launches are staged
+@pytest.mark.parametrize("elem,nx,nodes,taken", [
+    (4, 1024, 1_499_999, "00"), (4, 1024, 1_500_000, "10"), (4, 1024, 2_200_000, "11"), (4, 60, 2_200_000, "11"),
+    (4, 192, 2_199_999, "10"), (4, 192, 2_200_000, "11"), (4, 128, 9_000_000, "10"), (4, 64, 1_500_000, "10"),
+    (4, 62, 9_000_000, "10"), (4, 30, 9_000_000, "00"), (4, 8, 9_000_000, "00"), (4, 2, 9_000_000, "00"),
+    (4, 255, 1_499_999, "00"), (4, 255, 1_500_000, "11"), (4, 99, 1_500_000, "11"), (4, 91, 1_500_000, "10"),
+    (4, 61, 9_000_000, "00"), (4, 31, 9_000_000, "00"), (4, 1, 9_000_000, "00"),
+    (8, 1024, 699_999, "00"), (8, 1024, 700_000, "11"), (8, 30, 700_000, "11"), (8, 96, 700_000, "11"),
+    (8, 64, 700_000, "10"), (8, 64, 1_100_000, "11"), (8, 32, 1_099_999, "00"), (8, 32, 1_100_000, "10"),
+    (8, 31, 1_100_000, "10"), (8, 8, 9_000_000, "00"), (8, 1, 9_000_000, "00"),
+    (2, 1024, 2_499_999, "00"), (2, 1024, 2_500_000, "11"), (2, 600, 2_500_000, "11"), (2, 190, 2_500_000, "10"),
+    (2, 40, 2_500_000, "10"), (2, 66, 9_000_000, "00"), (2, 30, 9_000_000, "00"), (2, 1025, 9_000_000, "00")])
+def test_where_two_iterations_per_launch_pay(rules, elem, nx, nodes, taken):
+    rules.rows_pay.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_longlong, ctypes.c_int, ctypes.c_int]
+    assert "".join(str(rules.rows_pay(elem, nx, nodes, mixed, 0)) for mixed in (0, 1)) == taken
+
+
+@pytest.mark.parametrize("nx,tile,nodes,taken", [
+    (512, 512, 2_499_999, "00"), (512, 512, 2_500_000, "10"), (480, 480, 2_500_000, "11"), (384, 384, 9_000_000, "11"),
+    (256, 512, 9_000_000, "00"), (256, 256, 9_000_000, "10"), (192, 384, 9_000_000, "00"), (192, 192, 9_000_000, "10"),
+    (128, 512, 9_000_000, "00"), (128, 256, 9_000_000, "00"), (64, 512, 9_000_000, "00")])
+def test_where_they_pay_against_staged_launches(rules, nx, tile, nodes, taken):
+    rules.rows_pay.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_longlong, ctypes.c_int, ctypes.c_int]
+    assert "".join(str(rules.rows_pay(2, nx, nodes, mixed, tile)) for mixed in (0, 1)) == taken
 
 
 @pytest.mark.parametrize("tile,nodes,pairs", [

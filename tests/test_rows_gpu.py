@@ -87,6 +87,38 @@ def test_graph_replays_of_two_iterations():
     assert np.allclose(out[0], out[1], rtol=0, atol=1e-6)
 
 
+# both sides of the rule, on flows with 0.2% and 10% of the nodes of another type (below and above 1% of the pairs
+# with one node that collides): the kernel that ran, and single launches' bits from both
+@pytest.mark.parametrize("precision,storage,nx,ny,p,two", [
+    ("fp32", "same", 1500, 1000, 0.002, True), ("fp32", "same", 1500, 1000, 0.1, False),
+    ("fp32", "same", 1450, 1531, 0.1, True), ("fp32", "same", 62, 24203, 0.002, True),
+    ("fp32", "same", 62, 40001, 0.1, False), ("fp32", "same", 30, 52001, 0.002, False),
+    ("fp32", "same", 192, 11461, 0.1, True), ("fp32", "same", 255, 5891, 0.1, True),
+    ("fp32", "same", 91, 17001, 0.1, False), ("fp64", "same", 1025, 684, 0.1, True),
+    ("fp64", "same", 64, 11001, 0.1, False), ("fp64", "same", 64, 17191, 0.1, True),
+    ("fp64", "same", 31, 40001, 0.002, True), ("fp64", "same", 31, 40001, 0.1, False),
+    ("fp32", "fp16s", 1922, 1302, 0.1, True), ("fp32", "bf16", 190, 13201, 0.002, True),
+    ("fp32", "bf16s", 190, 13201, 0.1, False), ("fp32", "fp16", 66, 38001, 0.002, False),
+    ("fp32", "bf16", 512, 4901, 0.002, True), ("fp32", "fp16s", 512, 4901, 0.1, False),
+    ("fp32", "fp16s", 256, 10000, 0.002, False), ("fp32", "fp16s", 256, 10301, 0.002, True)])
+def test_where_two_iterations_run(precision, storage, nx, ny, p, two):
+    fl = random_flags("d2q9", (1, ny, nx), TYPES[:4], zones=2, seed=nx, p_type=p)
+    fl[(fl & BOUNDARY) == SOLID] = SOLID  # no collision there
+    out = []
+    for cuts in ([1] * 5, [5]):
+        g = start(nx, ny, precision, storage, fl, ny)
+
+        def run():
+            for n in cuts:
+                g.Iterate(n, M.ITER_NORM)
+            g.sync()
+
+        assert ("k_iterate_rows" in kernels(run)) == (two and cuts == [5])
+        out.append(g.save().tobytes())
+        g.close()
+    assert out[0] == out[1]
+
+
 # 16-bit rows that can be staged: in pairs while the lattice stays in L2, staged beyond, the same bits
 @pytest.mark.parametrize("nx,ny,kernel", [(256, 8202, "k_iterate_pair"), (256, 8204, "k_iterate_tma"),
                                           (256, 10155, "k_iterate_pair"), (256, 10157, "k_iterate_tma"),
@@ -102,6 +134,41 @@ def test_single_launches_of_staged_widths(nx, ny, kernel):
         out.append(g.save().tobytes())
         g.close()
     assert out[0] == out[1] == out[2]
+
+
+# the choice follows the node types: captured launches of the other kernel are dropped
+def test_node_types_that_change_the_choice():
+    nx, ny = 1500, 1010
+    clean, porous = (random_flags("d2q9", (1, ny, nx), ["Solid"], seed=3, p_type=p) for p in (0.0, 0.1))
+    porous[(porous & BOUNDARY) == SOLID] = SOLID
+    out = []
+    for cuts in ([40], [1] * 40):
+        g = start(nx, ny, "fp32", "same", clean, 1)
+        ran = []
+        for fl in (clean, porous, clean):
+            g.set_flags(fl)
+            ran.append("k_iterate_rows" in kernels(lambda: ([g.Iterate(n, M.ITER_NORM) for n in cuts], g.sync())))
+        assert ran == ([True, False, True] if cuts == [40] else [False] * 3)
+        out.append(g.save().tobytes())
+        g.close()
+    assert out[0] == out[1]
+
+
+@pytest.mark.parametrize("precision,storage,nx,ny", [
+    ("fp32", "same", 1500, 1010), ("fp64", "same", 1024, 700), ("fp32", "fp16s", 1920, 1304)])
+def test_graph_replays_equal_single_launches(precision, storage, nx, ny):
+    """More iterations than a graph holds, in one call and one by one, bit for bit from a flow."""
+    fl = random_flags("d2q9", (1, ny, nx), TYPES[:4], zones=2, seed=5, p_type=0.002)
+    out = []
+    for cuts in ([1] * 75, [75]):
+        g = start(nx, ny, precision, storage, fl, 2)
+        for n in cuts:
+            g.Iterate(n, M.ITER_NORM)
+        u = g.GetQuantity("U")
+        assert np.isfinite(u).all() and np.abs(u).max() > 1e-3
+        out.append(g.save().tobytes())
+        g.close()
+    assert out[0] == out[1]
 
 
 # iterations per replay even, odd and one; iteration counts that end anywhere in
