@@ -53,7 +53,8 @@ struct LaunchTables {
   int* err;                    // set by a staging wait that ran out
   const BatchRow* rows;        // strip segments of the cases that advance two iterations per launch
   const int* nrows;
-  int nrows_grid;              // > 0: two iterations per launch, in this many blocks
+  int nrows_grid;              // two iterations per launch, in this many blocks
+  int two;                     // for the cases that rows_case takes with this; 0: none
   int odd_grid;                // tiles of those cases: their single plain iteration
   const BatchTile* odd_tiles;
   const int* nodd;
@@ -77,12 +78,12 @@ struct BatchImpl {
   // the derived constants k of a case from its settings (host, in real_t)
   void (*derive)(BatchCase&);
   void (*clear)(BatchCase*, int n, int K, cudaStream_t);
-  void (*advance)(BatchCase*, int n, int K, bool two, cudaStream_t);
+  void (*advance)(BatchCase*, int n, int K, int two, cudaStream_t);
   void (*init)(const BatchCase&, const void* dst, cudaStream_t, int bx, int by);
   void (*quantity)(const BatchCase&, int parity, int q, int vec, double scale, void* out, cudaStream_t);
   int (*blocks_per_sm)(int threads);
   const void* (*tile_kernel)(int which);  // 0 one-tile plain, 1 one-tile Globals, 2 pair, 3 one-tile odd, 4 rows
-  bool (*takes_rows)(int nx);             // two iterations per launch possible for a case of this width
+  bool (*takes_rows)(int nx, int tile);   // two iterations per launch for cases of this width (rows_case)
   int pair_threads;                        // block-size limit of the pair kernel; 0: no pair kernel
   bool group_staging;                      // staged cases must share their settings (packed collision)
   // smallest staged tile (nodes) of a case; cases with smaller tiles take the
@@ -124,7 +125,7 @@ struct BL {
     const dim3 b(bx, block_rows(bx, by, 256));
     const BatchCase* c = L.cases;
     const BatchTile* t = L.tiles;
-    const bool two = L.nrows_grid > 0;
+    const int two = L.two;
     if constexpr (rows) {
       if (two) {
         if (k % 2 == 1)
@@ -188,8 +189,8 @@ struct BL {
     return which ? reinterpret_cast<const void*>(k_iterate_batch_tile<M, R, St, ROLE_GLOBALS>)
                  : reinterpret_cast<const void*>(k_iterate_batch_tile<M, R, St, ROLE_PLAIN>);
   }
-  static bool takes_rows(int nx) { return rows && rows_case<R>(nx); }
-  static void advance(BatchCase* c, int n, int K, bool two, cudaStream_t s) {
+  static bool takes_rows(int nx, int tile) { return rows && rows_case(sizeof(R) == 4, nx, tile); }
+  static void advance(BatchCase* c, int n, int K, int two, cudaStream_t s) {
     k_batch_advance<R><<<(n + 127) / 128, 128, 0, s>>>(c, n, K, two);
   }
   // resident blocks per SM of the plain kernel at this block size
@@ -326,7 +327,7 @@ struct tclb_batch {
   BatchRow* d_rows = nullptr;
   BatchTile* d_odd = nullptr;
   size_t tiles_cap = 0, ttiles_cap = 0, rows_cap = 0, odd_cap = 0;
-  bool two = false;
+  int two = 0;  // argument of rows_case for these cases; 0: none
   int nrows = 0, nodd = 0;
   std::vector<BatchCase> cases;
   std::vector<size_t> bytes;
@@ -350,7 +351,7 @@ struct tclb_batch {
   std::vector<cudaGraphNode_t> glob_nodes;   // the Globals launch
   std::vector<cudaGraphNode_t> odd_nodes, rows_nodes;  // of the cases that advance two iterations per launch
   int graph_grid[4] = {0, 0, 0, 0};          // their grids in the instantiated graph
-  int graph_key[9] = {-1, -1, -1, -1, -1, -1, -1, -1, -1};
+  int graph_key[10] = {-1, -1, -1, -1, -1, -1, -1, -1, -1, -1};
   ReadBack read_back;
   int paths = TCLB_LAUNCH_PAIRS | TCLB_LAUNCH_TMA | TCLB_BATCH_ADAPTIVE;  // tclb_batch_set_paths
 };
@@ -462,15 +463,20 @@ void update_staging(tclb_batch* B) {
 }
 
 // Two iterations per launch for the cases k_iterate_batch_rows takes, where
-// they have nodes enough for it to be faster (the one-lattice rule).
-bool rows_case_of(const tclb_batch* B, size_t s) { return B->two && B->I->takes_rows(B->cases[s].nx); }
+// they have nodes enough for it to be faster (rows_case).
+bool rows_case_of(const tclb_batch* B, size_t s) { return B->two && B->I->takes_rows(B->cases[s].nx, B->two); }
 void update_two(tclb_batch* B) {
-  size_t n = 0;
+  B->two = 0;
+  if (B->user_grid != 0 || B->K < 2) return;
+  size_t all = 0, wide = 0;
   for (size_t s = 0; s < B->cases.size(); s++) {
     const BatchCase& C = B->cases[s];
-    if (live(B, s) && B->I->takes_rows(C.nx)) n += (size_t)C.nx * C.ny;
+    if (!live(B, s)) continue;
+    if (B->I->takes_rows(C.nx, ROWS_ALL)) all += (size_t)C.nx * C.ny;
+    if (B->I->takes_rows(C.nx, B->bx)) wide += (size_t)C.nx * C.ny;
   }
-  B->two = B->user_grid == 0 && B->K >= 2 && n >= rows_min_nodes(B->elem);
+  const size_t least = rows_min_nodes(B->elem);
+  if (wide >= least) B->two = all - wide < least ? ROWS_ALL : B->bx;
 }
 
 int rebuild_tiles(tclb_batch* B) {
@@ -560,8 +566,8 @@ int ensure_graph(tclb_batch* B) {
       std::string(reinterpret_cast<const char*>(B->group.data()), B->group.size() * sizeof(double)));
   // with two iterations per launch: whether cases of one remain
   const int forms = B->two ? (B->nplain > 0 ? 2 : 1) : 0;
-  const int key[9] = {B->bx, B->by, B->K, (int)B->cases.size(), B->user_grid, B->paths, has_tma, group_hash, forms};
-  if (B->graph && std::equal(key, key + 9, B->graph_key)) return update_graph_grid(B);
+  const int key[10] = {B->bx, B->by, B->K, (int)B->cases.size(), B->user_grid, B->paths, has_tma, group_hash, forms, B->two};
+  if (B->graph && std::equal(key, key + 10, B->graph_key)) return update_graph_grid(B);
   if (B->graph) {
     cudaGraphExecDestroy(B->graph);
     B->graph = nullptr;
@@ -584,7 +590,7 @@ int ensure_graph(tclb_batch* B) {
   const int grid_all = per_tile ? std::max(1, B->ntiles) : B->grid_blocks;
   const int form = !per_tile ? FORM_PERSISTENT : (pair_form(B) ? FORM_PAIR : FORM_TILE);
   const LaunchTables L = {B->d_cases, B->d_tiles, B->d_ntiles, B->d_ttiles, B->d_ntiles + 2, B->d_err, B->d_rows,
-                          B->d_ntiles + 4, B->two ? rows_grid(B) : 0, std::max(1, B->nodd), B->d_odd, B->d_ntiles + 3};
+                          B->d_ntiles + 4, rows_grid(B), B->two, std::max(1, B->nodd), B->d_odd, B->d_ntiles + 3};
   cudaGraph_t g;
   BCK(cudaStreamBeginCapture(B->stream, cudaStreamCaptureModeThreadLocal));
   const int n = (int)B->cases.size();
@@ -631,7 +637,7 @@ int ensure_graph(tclb_batch* B) {
   B->graph_grid[1] = grid_all;
   B->graph_grid[2] = L.odd_grid;
   B->graph_grid[3] = rows_grid(B);
-  std::copy(key, key + 9, B->graph_key);
+  std::copy(key, key + 10, B->graph_key);
   return TCLB_OK;
 }
 

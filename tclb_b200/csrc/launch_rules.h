@@ -107,4 +107,24 @@ inline bool pairs_pay_2d(std::size_t nodes, int tile) {
   return tile < 192 || nodes < (tile >= 320 ? 2100000u : 2600000u);
 }
 
+// Whether the cases nx wide of a batch with tiles `tile` columns wide take them
+// (with rows_min_nodes nodes in such cases together: FP32 cases of 256^2, 10%
+// solid, 15.0/16.7 us an iteration of the batch at 1.0 M nodes, 25.6/25.7 at
+// 1.6 M, 60.7/51.3 at 4.0 M). FP64: every width (the least gain, 32 wide on
+// tiles of 32: 1.0 M nodes 36.3/27.6, 10% solid 39.0/32.8). FP32: even
+// widths whose strips have at most 1.5 times the lanes of the tiles, which have
+// idle lanes too (clean and 10% solid, tiles of 64, 1.6 M nodes: 48 wide
+// 32.2/18.7 and 34.3/26.4, 96 28.0/18.5 and 29.2/26.2, 128 24.9/18.4 and
+// 25.9/27.7, 256 24.9/16.7 and 25.6/25.7; 64 wide, twice the lanes, 25.1/23.3
+// and 26.0/33.8), or every even width (tile = ROWS_ALL) where those left over
+// have fewer than rows_min_nodes nodes: launches of their own, two for each of
+// the others, would cost the batch more (three each of 64 x 16 to 2048 x 512,
+// 2% solid: 49.8/43.8).
+constexpr int ROWS_ALL = 1 << 20;
+constexpr bool rows_case(bool pair, int nx, int tile) {
+  if (!pair) return true;
+  const long long strips = (nx - 1) / rows_columns(true, 2) + 1, tiles = (nx - 1) / tile + 1;
+  return nx % 2 == 0 && 2 * strips * rows_lanes(true) <= 3 * tiles * tile;
+}
+
 }  // namespace tclb

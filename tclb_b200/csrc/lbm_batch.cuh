@@ -131,18 +131,14 @@ __device__ __forceinline__ CaseTwos case_twos(const BatchCase& C, int K) {
   const int plain = d - (glob ? 1 : 0);
   return {plain / 2, (plain & 1) != 0, glob};
 }
-// Whether k_iterate_batch_rows takes a case of width nx: pairs need an even
-// width, FP64 has one node per lane.
-template <class R>
-__host__ __device__ constexpr bool rows_case(int nx) { return sizeof(R) == 8 || nx % 2 == 0; }
-
 // What a launch of the one-node kernels runs: launch k of K of the cases that
-// advance one iteration per launch (`two`: not those of k_iterate_batch_rows),
+// advance one iteration per launch (with `two`, the argument of rows_case, not
+// those that k_iterate_batch_rows takes),
 // the single plain iteration of the others, or the Globals iteration of all.
 enum BatchRole { ROLE_PLAIN, ROLE_ODD, ROLE_GLOBALS };
 template <class R, BatchRole ROLE>
-__device__ __forceinline__ bool case_on(const BatchCase& C, int k, int K, bool two, int& parity) {
-  if (two && rows_case<R>(C.nx)) {
+__device__ __forceinline__ bool case_on(const BatchCase& C, int k, int K, int two, int& parity) {
+  if (two && rows_case(sizeof(R) == 4, C.nx, two)) {
     const CaseTwos t = case_twos(C, K);
     parity = (C.flips + t.twos + (ROLE == ROLE_GLOBALS && t.odd ? 1 : 0)) & 1;
     return ROLE == ROLE_ODD ? t.odd : (ROLE == ROLE_GLOBALS && t.glob);
@@ -219,7 +215,7 @@ __global__ void __launch_bounds__(256) k_iterate_batch(const BatchCase* __restri
 template <class M, class R, BatchRole ROLE>
 __device__ __forceinline__ bool batch_tile_args(const BatchCase* __restrict__ cases,
                                                 const BatchTile* __restrict__ tiles, const int* __restrict__ ntiles_p,
-                                                int k, int K, bool two, BatchTile& tile, Args<R, M::NSET>& a) {
+                                                int k, int K, int two, BatchTile& tile, Args<R, M::NSET>& a) {
   const int t = blockIdx.x;
   if (t >= *ntiles_p) return false;
   tile = tiles[t];
@@ -236,7 +232,7 @@ __device__ __forceinline__ bool batch_tile_args(const BatchCase* __restrict__ ca
 template <class M, class R, class St, BatchRole ROLE>
 __global__ void __launch_bounds__(256, (ROLE == ROLE_GLOBALS || sizeof(R) == 8) ? 1 : M::BATCH_MIN_BLOCKS)
     k_iterate_batch_tile(const BatchCase* __restrict__ cases, const BatchTile* __restrict__ tiles,
-                         const int* __restrict__ ntiles_p, int k, int K, bool two) {
+                         const int* __restrict__ ntiles_p, int k, int K, int two) {
   constexpr bool G = ROLE == ROLE_GLOBALS;
   BatchTile tile;
   Args<R, M::NSET> a;
@@ -272,7 +268,7 @@ __global__ void __launch_bounds__(M::PAIR_THREADS, M::PAIR_MIN_BLOCKS)
                          const int* __restrict__ ntiles_p, int k, int K) {
   BatchTile tile;
   Args<R, M::NSET> a;
-  if (!batch_tile_args<M, R, ROLE_PLAIN>(cases, tiles, ntiles_p, k, K, false, tile, a)) return;
+  if (!batch_tile_args<M, R, ROLE_PLAIN>(cases, tiles, ntiles_p, k, K, 0, tile, a)) return;
   using T = typename St::T;
   const StrideAddr<T> P{static_cast<const T*>(a.src), static_cast<T*>(a.dst), a.stride};
   const int z = tile.z;
@@ -483,12 +479,12 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32, sizeof(R) == 8 ? 4 : 5)  // t
 
 // End of a replay: counters and remaining iterations of every active case.
 template <class R>
-__global__ void k_batch_advance(BatchCase* cases, int ncases, int K, bool two) {
+__global__ void k_batch_advance(BatchCase* cases, int ncases, int K, int two) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= ncases || !cases[c].active) return;
   const int r = cases[c].remaining;
   const int d = r < K ? r : K;
-  if (two && rows_case<R>(cases[c].nx)) {
+  if (two && rows_case(sizeof(R) == 4, cases[c].nx, two)) {
     const CaseTwos t = case_twos(cases[c], K);
     cases[c].flips += t.twos + (t.odd ? 1 : 0) + (t.glob ? 1 : 0);
   } else {

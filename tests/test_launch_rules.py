@@ -21,6 +21,7 @@ extern "C" int rows_pay(int elem, int nx, long long nodes, int mixed, int tile) 
   return tclb::rows_pay(elem, nx, nodes, mixed != 0, tile);
 }
 extern "C" int pairs_pay_2d(long long nodes, int tile) { return tclb::pairs_pay_2d(nodes, tile); }
+extern "C" int rows_case(int pair, int nx, int tile) { return tclb::rows_case(pair != 0, nx, tile); }
 """
 
 
@@ -95,6 +96,15 @@ def test_where_they_pay_against_staged_launches(rules, nx, tile, nodes, taken):
 def test_pairs_or_staged_single_launches(rules, tile, nodes, pairs):
     rules.pairs_pay_2d.argtypes = [ctypes.c_longlong, ctypes.c_int]
     assert rules.pairs_pay_2d(nodes, tile) == pairs
+
+
+# widths at which the tiles have 1, 1.5 and 2 times fewer lanes than the strips, or more
+@pytest.mark.parametrize("nx,tile,pairs", [
+    (32, 32, 0), (32, 64, 1), (48, 64, 1), (60, 64, 1), (62, 64, 0), (64, 64, 0), (64, 128, 1), (66, 64, 1),
+    (96, 32, 1), (128, 64, 1), (128, 128, 1), (192, 64, 1), (1024, 64, 1), (63, 64, 0), (1, 32, 0), (2, 32, 0),
+    (2, 1 << 20, 1), (64, 1 << 20, 1), (63, 1 << 20, 0), (1 << 21, 1 << 20, 1), ((1 << 31) - 2, 1 << 20, 1)])
+def test_cases_of_a_batch_with_two_iterations_per_launch(rules, nx, tile, pairs):
+    assert rules.rows_case(1, nx, tile) == pairs and rules.rows_case(0, nx, tile) == 1
 
 
 @pytest.mark.gpu

@@ -203,3 +203,36 @@ def test_batch_of_two_iterations_per_launch(precision, K, at_end):
         assert np.allclose(b.globals(cid), g.globals, rtol=1e-6 if precision == "fp32" else 1e-9, atol=1e-9)
         g.close()
     b.close()
+
+
+# widths that strips fit and that they do not, even and odd, in one batch; nodes enough for two iterations per launch,
+# and not enough; in FP32 the narrow cases with nodes enough for launches of their own, and without
+@pytest.mark.parametrize("precision,shapes,two,one", [
+    ("fp32", [(1000, 1500), (97, 64), (41, 128), (33, 32), (40, 66)], True, False),
+    ("fp32", [(1000, 1500), (97, 64), (41, 128), (55, 301), (33, 32), (40, 66)], True, True),
+    ("fp32", [(1000, 1500), (23500, 64), (41, 128)], True, True),
+    ("fp32", [(1000, 1300), (23500, 64), (41, 128)], False, True),
+    ("fp64", [(1000, 700), (97, 64), (55, 301), (33, 32)], True, False),
+    ("fp64", [(1000, 640), (97, 64), (55, 301)], False, True)])
+def test_which_cases_of_a_batch_take_two_iterations(precision, shapes, two, one):
+    b = Batch("d2q9", precision, budget_bytes=8 << 30)
+    b.set_launch(64, 16, 5)
+    specs = [CaseSpec(random_flags("d2q9", (1,) + sh, TYPES[:2], seed=k, p_type=0.05),
+                      {"Viscosity": 0.05, "GravitationX": 1e-5}, {0: {"VelocityX": 0.02}}, 12)
+             for k, sh in enumerate(shapes)]
+    ids = [b.add_case(s) for s in specs]
+    ran = kernels(b.step)
+    assert ("k_iterate_batch_rows" in ran) == two
+    assert ("BatchRole)0" in ran) == one, ran  # ROLE_PLAIN: one iteration per launch
+    b.run_to_completion()
+    for cid, s in zip(ids, specs):
+        assert b.poll(cid) == (s.niter, 0)
+        ny, nx = s.flags.shape[1:]
+        g = Lattice("d2q9", nx, ny, precision=precision)
+        g.set_flags(s.flags)
+        apply_params(g, [("setting", "Viscosity", 0.05), ("setting", "GravitationX", 1e-5), ("zone", "VelocityX", 0.02, 0)])
+        g.Init()
+        g.Iterate(s.niter, M.ITER_NORM | M.ITER_LASTGLOB)
+        assert np.array_equal(b.quantity(cid, "U"), g.GetQuantity("U")), (nx, ny)
+        g.close()
+    b.close()
