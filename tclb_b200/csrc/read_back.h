@@ -51,7 +51,7 @@ class ReadBackPool {
     cudaError_t e = cudaStreamSynchronize(s);  // the parts are copied on streams of their own
     if (e != cudaSuccess) return e;
     const size_t n = lanes_.size(), part = ((bytes + n - 1) / n + 4095) / 4096 * 4096;
-    std::vector<cudaError_t> err(n, cudaSuccess);
+    cudaError_t err[MAX_LANES] = {};
     std::vector<std::thread> threads;
     auto run = [&](size_t k, bool own) {  // own: in a thread of its own, whose current device is not set
       const size_t at = std::min(k * part, bytes), end = std::min(at + part, bytes);
@@ -74,6 +74,7 @@ class ReadBackPool {
 
  private:
   static constexpr size_t PARALLEL_BYTES = (size_t)4 << 20, FIRST_BYTES = (size_t)16 << 20, CHUNK = (size_t)512 << 10;
+  static constexpr unsigned MAX_LANES = 8;
   struct Lane {
     char* buf[2] = {nullptr, nullptr};  // in buffers_
     cudaEvent_t event[2] = {nullptr, nullptr};
@@ -106,7 +107,7 @@ class ReadBackPool {
 
   bool prepare(int device) {
     if (!lanes_.empty()) return device == device_;
-    const size_t n = std::max(1u, std::min(8u, std::thread::hardware_concurrency() / 2));
+    const size_t n = std::max(1u, std::min(MAX_LANES, std::thread::hardware_concurrency() / 2));
     try {
       lanes_.resize(n);
     } catch (const std::exception&) {
