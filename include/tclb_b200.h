@@ -290,8 +290,8 @@ int tclb_batch_get_launch(tclb_batch_h b, int* bx, int* by, int* iters_per_launc
 /* Paths of the plain launches: TCLB_LAUNCH_PAIRS (on by default) lets 16-bit
    storage update two neighbouring nodes per thread with 32-bit accesses when
    the tile width bx is a multiple of 64 and the grid is one block per tile
-   (blocks of bx / 2 x min(by, T / (bx / 2)) threads, T = 256, 128 for
-   d3q27_cumulant); the Globals launch keeps the one-node kernel.
+   (blocks of bx / 2 x min(by, T / (bx / 2)) threads, T = 256 for d2q9, 128
+   for the 3D models); the Globals launch keeps the one-node kernel.
    TCLB_LAUNCH_TMA (on by default) runs the plain launches of each 16-bit case
    whose rows fit the tile-staged kernel (nx a multiple of 32 up to 512) through
    it, tensor maps kept with the case;

@@ -1368,7 +1368,7 @@ __global__ void k_count_mixed_pairs(const flag_t* __restrict__ flags, unsigned n
 }
 
 // Block (32, M::PAIR_THREADS / 32): each warp covers 64 consecutive x of one
-// row. Plain iterations only (Globals iterations use k_iterate).
+// row. Plain iterations only (Globals iterations use k_iterate_globals).
 template <class M, class R, class St>
 __global__ void __launch_bounds__(M::PAIR_THREADS, M::PAIR_MIN_BLOCKS)
     k_iterate_pair(const Args<R, M::NSET> a, const PlaneAddr<typename St::T, M::Q> P) {

@@ -8,7 +8,8 @@
 // update of the row below, T stages deep. What stage k+1 needs of stage k is
 // held in registers -- of the populations with e_y = 0 the last row, of those
 // with e_y = +1 the last two, those with e_y = -1 are used at once -- and moves
-// in x by warp shuffles. No shared memory, no barrier, and nothing is
+// in x by warp shuffles. Only the source rows ahead pass through shared memory,
+// each warp's own (cp.async, one __syncwarp a row). Nothing is
 // exchanged between warps: every stage loses one column at each edge of the
 // strip, so strips overlap, and a segment of H output rows runs 2(T-1) rows
 // more through its first stage.
@@ -30,6 +31,7 @@ constexpr int ROWS_AHEAD = 2;   // rows staged ahead of the one updated
 // 4096 x 1024: 8 rows 33.3 us an iteration, 16 36.3, 32 47.4; 4096 x 4096:
 // 115, 120, 132).
 constexpr int ROWS_HEIGHT = 8;
+
 // A lane's one or two nodes of a population as stored.
 template <class St>
 struct RowPair {  // 16-bit storage: two values in a word
