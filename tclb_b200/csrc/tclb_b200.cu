@@ -395,7 +395,8 @@ struct Launch {
       // than 256 (one-row tiles, six consumer warps per block; porous 384 x 192 x
       // 192 213 / 274), tiles of fewer than 448 nodes (192^3 109 / 141), fewer than
       // four tiles per resident block (64^3 4.8 / 9.4; 128^3, at fourteen, 35.3 /
-      // 36.1; 256^3 256 / 246).
+      // 36.1, level; 256^3 256 / 246). Other multiples of 32 stay staged: the pair
+      // kernel of flat indexes was not measured there.
       if constexpr (M::identity_lanes)
         L->tma_pref_pairs = L->nx % 64 == 0 && (tma_wide(L->nx) || rows * L->nx < 448 || tiles < 4 * per_sm * sms);
       else if constexpr (M::DIM == 2)
